@@ -87,6 +87,8 @@ struct bm3d_b200_batch {
     unsigned long long *d_end = nullptr;  // [nclips]
     std::vector<unsigned> remaining_init;
     size_t match_smem = 0;
+    int kt = 9;          // temporal strip width, and
+    bool small = false;  // two-entry temporal lists (choose_match_form)
     cudaStream_t cap = nullptr;
     cudaGraphExec_t exec = nullptr;
 };
@@ -127,9 +129,27 @@ void release_device(bm3d_b200_batch *b) {
     b->prepared = false;
 }
 
-MatchGeometry clip_geometry(const bm3d_b200_batch *b, const BatchClip &c, int wx, int K) {
+MatchGeometry clip_geometry(const bm3d_b200_batch *b, const BatchClip &c) {
     return match_geometry_with(c.w, c.h, c.prm.block_step[0], c.prm.bm_range[0], c.prm.radius,
-                               c.prm.ps_range[0], wx, K);
+                               c.prm.ps_range[0], b->wx, b->K, b->small ? b->kt : b->K, b->small);
+}
+
+// The matching kernel's form for the batch's clips at its CTA width and strip:
+// two-entry temporal lists where every clip allows them and its tile fits,
+// with the temporal strip width that suits most temporal candidates.
+void choose_match_form(bm3d_b200_batch *b) {
+    double work[2] = {};  // of clips whose temporal windows suit strips of 9, of 11
+    b->small = true;
+    for (const BatchClip &c : b->clips) {
+        b->small &= c.prm.radius == 0 || c.prm.ps_num[0] <= 2;
+        const double wt = 2 * c.prm.ps_range[0] + 1;
+        work[temporal_strip_width(c.prm.ps_range[0]) == 11] +=
+            (double)c.n * c.w * c.h * c.prm.radius * wt * wt /
+            (c.prm.block_step[0] * c.prm.block_step[0]);
+    }
+    b->kt = work[1] > work[0] ? 11 : 9;
+    for (const BatchClip &c : b->clips)
+        b->small &= clip_geometry(b, c).smem <= kMatchSmemMax;
 }
 
 // Stage tables of one clip (fused VAggregate mapping, source/source.cpp:830-844).
@@ -173,14 +193,19 @@ int prepare(bm3d_b200_batch *b) {
     std::vector<long long> off(6 * (nc + 1), 0);
     b->remaining_init.assign(nc, 0);
     b->match_smem = 0;
+    choose_match_form(b);
     for (int i = 0; i < nc; ++i) {
         BatchClip &c = b->clips[i];
         const int N = c.n, tw = 2 * c.prm.radius + 1;
         const size_t ntab = (size_t)N * tw, plane = (size_t)c.h * c.stride;
-        const MatchGeometry g = clip_geometry(b, c, b->wx, b->K);
-        if (g.smem > 220 * 1024)
+        MatchGeometry g = clip_geometry(b, c);
+        choose_pitches(g, c.prm.block_step[0], c.prm.bm_range[0], c.prm.radius, c.prm.ps_range[0]);
+        const size_t range_bytes =
+            match_range_bytes(c.prm.block_step[0], c.prm.bm_range[0], c.prm.radius,
+                              c.prm.ps_range[0], b->wx, b->K);
+        if (range_bytes > kMatchSmemLimit)
             return bfail(BM3D_B200_ERR_UNSUPPORTED, "BM3D batch: clip %d needs %zu B of shared memory",
-                         i, g.smem);
+                         i, range_bytes);
         b->match_smem = std::max(b->match_smem, g.smem);
         if (!c.d_basic) {
             BTRY(cudaMalloc(&c.d_basic, (size_t)N * plane * sizeof(float)));
@@ -284,7 +309,7 @@ int enqueue_match(bm3d_b200_batch *b, int st, unsigned long long *counter,
                   unsigned long long *stamp, cudaStream_t s) {
     const int nc = (int)b->clips.size();
     MatchBatch mb{b->d_mp + st * nc, b->d_off + (st * 3 + 0) * (nc + 1), nc, counter, stamp};
-    BTRY(launch_match_batch(mb, b->K, b->wx, b->match_smem, s));
+    BTRY(launch_match_batch(mb, b->K, b->kt, b->small, b->wx, b->match_smem, s));
     return BM3D_B200_OK;
 }
 

@@ -72,8 +72,7 @@ int check_search(int width, int height, int stride, int block_step, int bm_range
     if (ps_num <= 0 || ps_num > 8)
         return fail(BM3D_B200_ERR_INVALID, "BM3D: \"ps_num\" must be in range [1, 8]");
     if (ps_range <= 0) return fail(BM3D_B200_ERR_INVALID, "BM3D: \"ps_range\" must be positive");
-    MatchGeometry g = match_geometry(width, height, block_step, bm_range, radius, ps_range);
-    if (g.smem > 220 * 1024)
+    if (match_too_large(block_step, bm_range, radius, ps_range))
         return fail(BM3D_B200_ERR_UNSUPPORTED,
                     "BM3D: search range too large for the on-chip tile (bm_range + radius * "
                     "ps_range = %d)",
@@ -265,7 +264,7 @@ static int graph_create_impl(bm3d_b200_graph **out, float *d_res, float *d_src, 
     g->metric = bm_error;
     g->tx2 = transform_2d;
     g->tx1 = transform_1d;
-    g->geo = match_geometry(width, height, block_step, bm_range, radius, ps_range);
+    g->geo = match_geometry(width, height, block_step, bm_range, radius, ps_num, ps_range);
 
     auto cleanup = [&](int rc) {
         bm3d_b200_graph_destroy(g);
@@ -852,7 +851,7 @@ extern "C" int bm3d_b200_clip_create(bm3d_b200_clip **out, int width, int height
                                   p.radius, p.ps_num[pq], p.ps_range[pq]))
             return cleanup(rc);
         c->geo[q] = match_geometry(c->pw[q], c->ph[q], p.block_step[pq], p.bm_range[pq], p.radius,
-                                   p.ps_range[pq]);
+                                   p.ps_num[pq], p.ps_range[pq]);
         max_blk = std::max(max_blk, (size_t)c->geo[q].nbx * c->geo[q].nby);
     }
     if (p.chroma) {
@@ -1427,7 +1426,7 @@ extern "C" int bm3d_b200_learned_match(const float *const *d_frames, const void 
     if (cells_spatial < 1 || cells_spatial > 8 || cells_temporal < 1 || cells_temporal > 8)
         return fail(BM3D_B200_ERR_INVALID, "BM3D: proposal cell counts must be in range [1, 8]");
     const int tw = 2 * radius + 1;
-    const MatchGeometry g = match_geometry(width, height, block_step, bm_range, radius, ps_range);
+    const MatchGeometry g = match_geometry(width, height, block_step, bm_range, radius, ps_num, ps_range);
     const MatchGeometry lg = learned_geometry(width, height, block_step, bm_range, radius,
                                               ps_range);
     if (lg.smem > 220 * 1024 || !learned_ordinals_fit(bm_range, ps_num, ps_range))
@@ -1621,7 +1620,7 @@ extern "C" int bm3d_b200_window_noalloc(float *d_res, const float *d_src, int wi
         return rc;
     if (!(sigma >= 0.0f) || !(sigma_u >= 0.0f) || !(sigma_v >= 0.0f))
         return fail(BM3D_B200_ERR_INVALID, "BM3D: \"sigma\" must be non-negative");
-    const MatchGeometry geo = match_geometry(width, height, block_step, bm_range, radius, ps_range);
+    const MatchGeometry geo = match_geometry(width, height, block_step, bm_range, radius, ps_num, ps_range);
     const size_t nblk = (size_t)geo.nbx * geo.nby;
     const size_t need = kNoallocTableBytes + nblk * 8 * sizeof(int);
     if (need > kNoallocScratchBytes)
@@ -2233,7 +2232,7 @@ extern "C" int bm3d_b200_stream_create(bm3d_b200_stream **out, int width, int he
         const bool matched = p.chroma ? q == 0 : s->process[q];
         if (!matched) continue;
         s->geo[q] = match_geometry(s->pw[q], s->ph[q], p.block_step[pq], p.bm_range[pq],
-                                   p.radius, p.ps_range[pq]);
+                                   p.radius, p.ps_num[pq], p.ps_range[pq]);
         s->max_blk = std::max(s->max_blk, (size_t)s->geo[q].nbx * s->geo[q].nby);
     }
     s->frame_floats = off;

@@ -486,6 +486,21 @@ __device__ __forceinline__ void list_insert(List8 &l, float err, int pos) {
     }
 }
 
+// list_insert into the first N entries, without branches (err below the N-th
+// entry's distance; with ties the earlier entry stays in front).
+template <int N>
+__device__ __forceinline__ void list_insert_n(List8 &l, float err, int pos) {
+#pragma unroll
+    for (int i = N - 1; i > 0; --i) {
+        const bool shift = err < l.e[i - 1];
+        const bool here = err < l.e[i];
+        l.e[i] = fmaxf(l.e[i - 1], fminf(l.e[i], err));
+        l.p[i] = shift ? l.p[i - 1] : (here ? pos : l.p[i]);
+    }
+    l.p[0] = err < l.e[0] ? pos : l.p[0];
+    l.e[0] = fminf(l.e[0], err);
+}
+
 // Register-array element at a runtime index without local-memory indexing.
 template <int N, typename T>
 __device__ __forceinline__ T pick(const T (&a)[N], int i) {

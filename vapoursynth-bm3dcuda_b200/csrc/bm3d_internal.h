@@ -53,6 +53,11 @@ struct MatchParams {
     int metric;      // block distance: 0 SSD; 1 SAD, 2 ZSSD, 3 ZSAD, 4 SSD/NORM
 };
 
+// Search ranges whose one-warp CTA needs more shared memory are refused.
+constexpr size_t kMatchSmemLimit = 220 * 1024;
+// Largest dynamic shared memory of a matching launch.
+constexpr size_t kMatchSmemMax = 227 * 1024;
+
 struct MatchGeometry {
     int nbx, nby;
     int ks, kt, nsub_s, nsub_t, extra_cols;
@@ -60,17 +65,38 @@ struct MatchGeometry {
     int pitch;
     int tile_rows;
     size_t smem;
+    bool small;  // temporal stages keep at most two entries per frame
+    // the CTA tile when 4 or 8 lanes share a reference block (launches too
+    // small to fill the GPU with one lane per block)
+    struct Split {
+        int pitch, tile_rows;
+        size_t smem;
+    } split[2];
 };
 
 MatchGeometry match_geometry(int width, int height, int block_step, int bm_range, int radius,
-                             int ps_range);
-// Geometry with a given CTA width (warps) and strip width K (autotuner).
+                             int ps_num, int ps_range);
+// Whether a search range is refused: its pixel tile does not fit on chip.
+bool match_too_large(int block_step, int bm_range, int radius, int ps_range);
+// Shared memory of the general kernel's CTA of `wx` warps with strips of K.
+size_t match_range_bytes(int block_step, int bm_range, int radius, int ps_range, int wx, int K);
+// Geometry with a given CTA width (warps) and strip widths (autotuner).
 MatchGeometry match_geometry_with(int width, int height, int block_step, int bm_range, int radius,
-                                  int ps_range, int wx, int K);
+                                  int ps_range, int wx, int ks, int kt, bool small);
+// Its shared-memory row pitches, and the tiles of the split launches.
+void choose_pitches(MatchGeometry &g, int block_step, int bm_range, int radius, int ps_range);
+// Strip width of the temporal windows (small geometries).
+int temporal_strip_width(int ps_range);
 // CTA tiles of one launch over nwin windows.
 long long match_tiles(const MatchGeometry &g, int nwin);
 cudaError_t launch_match(const MatchParams &p, const MatchGeometry &g, int nwin,
                          cudaStream_t stream);
+// The same with `lanes` (1, 4, 8) lanes per reference block; launch_match_pairs
+// is its part for small geometries.
+cudaError_t launch_match_split(const MatchParams &p, const MatchGeometry &g, int nwin, int lanes,
+                               cudaStream_t stream);
+cudaError_t launch_match_pairs(const MatchParams &p, const MatchGeometry &g, int nwin, int lanes,
+                               cudaStream_t stream);
 
 // Learned block matching (bm3d_learned.cu): candidate cells ranked by the
 // proposer's embeddings, the best ones scored exactly; blocks whose best
@@ -117,7 +143,8 @@ struct MatchBatch {
     unsigned long long *counter;   // work counter, zero at launch
     unsigned long long *start_ns;  // globaltimer stamp of the first tile
 };
-cudaError_t launch_match_batch(const MatchBatch &b, int K, int wx, size_t smem,
+// K, kt: strip widths; small: every clip has ps_num <= 2 or radius 0
+cudaError_t launch_match_batch(const MatchBatch &b, int K, int kt, bool small, int wx, size_t smem,
                                cudaStream_t stream);
 
 // Collaborative filtering + scatter of one plane over a batch of windows.
