@@ -79,6 +79,7 @@ struct bm3d_b200_batch {
     // device descriptor arrays
     MatchParams *d_mp = nullptr;       // [2][nclips]
     FilterParams *d_fp = nullptr;      // [2][nclips]
+    CUtensorMap *d_maps = nullptr;     // [2][nclips] scatter maps, or null
     AggregateParams *d_ap = nullptr;   // [2][nclips]
     long long *d_off = nullptr;        // [6][nclips + 1]
     unsigned long long *d_ctr = nullptr;  // [kCounters]
@@ -112,6 +113,7 @@ void release_device(bm3d_b200_batch *b) {
     b->exec = nullptr;
     cudaFree(b->d_mp);
     cudaFree(b->d_fp);
+    cudaFree(b->d_maps);
     cudaFree(b->d_ap);
     cudaFree(b->d_off);
     cudaFree(b->d_ctr);
@@ -121,6 +123,7 @@ void release_device(bm3d_b200_batch *b) {
     b->d_remaining_init = nullptr;
     b->d_mp = nullptr;
     b->d_fp = nullptr;
+    b->d_maps = nullptr;
     b->d_ap = nullptr;
     b->d_off = nullptr;
     b->d_ctr = nullptr;
@@ -190,6 +193,8 @@ int prepare(bm3d_b200_batch *b) {
     std::vector<MatchParams> mp(2 * nc);
     std::vector<FilterParams> fp(2 * nc);
     std::vector<AggregateParams> ap(2 * nc);
+    std::vector<CUtensorMap> maps(2 * nc);
+    bool mapped = true;
     std::vector<long long> off(6 * (nc + 1), 0);
     b->remaining_init.assign(nc, 0);
     b->match_smem = 0;
@@ -261,6 +266,8 @@ int prepare(bm3d_b200_batch *b) {
             f.nbx = g.nbx;
             f.nwin = N;
             f.corner_weight = 1;
+            set_acc_pairs(f, c.d_acc, N, c.h);
+            mapped &= scatter_map(f, &maps[st * nc + i]);
             f.sigma = sig[st];
             f.extractor = c.prm.extractor_exp ? std::ldexp(1.0f, c.prm.extractor_exp) : 0.0f;
             AggregateParams &a = ap[st * nc + i];
@@ -288,6 +295,11 @@ int prepare(bm3d_b200_batch *b) {
         for (int i = 0; i < nc; ++i) off[s * (nc + 1) + i + 1] += off[s * (nc + 1) + i];
     BTRY(cudaMalloc(&b->d_mp, mp.size() * sizeof(MatchParams)));
     BTRY(cudaMalloc(&b->d_fp, fp.size() * sizeof(FilterParams)));
+    if (mapped) {
+        BTRY(cudaMalloc(&b->d_maps, maps.size() * sizeof(CUtensorMap)));
+        BTRY(cudaMemcpy(b->d_maps, maps.data(), maps.size() * sizeof(CUtensorMap),
+                        cudaMemcpyHostToDevice));
+    }
     BTRY(cudaMalloc(&b->d_ap, ap.size() * sizeof(AggregateParams)));
     BTRY(cudaMalloc(&b->d_off, off.size() * sizeof(long long)));
     BTRY(cudaMalloc(&b->d_ctr, kCounters * sizeof(unsigned long long)));
@@ -326,7 +338,7 @@ int enqueue_all(bm3d_b200_batch *b, cudaStream_t s) {
         // stage's first tile writes the spare slot
         if (int rc = enqueue_match(b, st, b->d_ctr + st * 3 + 0, b->d_ctr + 6 + st, s)) return rc;
         FilterBatch fb{b->d_fp + st * nc, b->d_off + (st * 3 + 1) * (nc + 1), nc,
-                       b->d_ctr + st * 3 + 1};
+                       b->d_ctr + st * 3 + 1, b->d_maps ? b->d_maps + st * nc : nullptr};
         BTRY(launch_filter_batch(fb, st == 1, s, b->filter_per_sm[st]));
         AggregateBatch ab{b->d_ap + st * nc, b->d_off + (st * 3 + 2) * (nc + 1), nc,
                           b->d_ctr + st * 3 + 2, st == 1 ? b->d_remaining : nullptr,
@@ -474,7 +486,8 @@ extern "C" int bm3d_b200_batch_autotune(bm3d_b200_batch *b, void *stream) {
         float best_t = FLT_MAX;
         int best_n = 0;
         for (int per_sm = 1; per_sm <= 4; ++per_sm) {
-            FilterBatch fb{b->d_fp + st * nc, b->d_off + (st * 3 + 1) * (nc + 1), nc, b->d_ctr};
+            FilterBatch fb{b->d_fp + st * nc, b->d_off + (st * 3 + 1) * (nc + 1), nc, b->d_ctr,
+                           b->d_maps ? b->d_maps + st * nc : nullptr};
             float t = 0;
             if (int rc = time_launch(
                     [&] { return launch_filter_batch(fb, st == 1, s, per_sm); }, &t))

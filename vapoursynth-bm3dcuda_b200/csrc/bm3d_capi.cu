@@ -743,6 +743,7 @@ int clip_run_impl(bm3d_b200_clip *c, const float *d_src, const float *d_ref, flo
             fp.nblk = g.nbx * g.nby;
             fp.nbx = g.nbx;
             fp.corner_weight = raw ? 0 : 1;
+            if (!raw) set_acc_pairs(fp, c->d_acc, N, Hq);
             fp.nwin = N;
             fp.sigma = sigma;
             fp.extractor = extractor_of(c->prm.extractor_exp);
@@ -1020,6 +1021,7 @@ int run_stage_windows(bm3d_b200_clip *c, void **d_tab, float *d_mult, bool final
     fp.win0 = w0;
     fp.nwin = w1 - w0;
     fp.corner_weight = 1;
+    set_acc_pairs(fp, final_ ? c->d_acc2 : c->d_acc, N, c->ph[0]);
     fp.sigma = final_ ? c->sigma_final[0] : c->sigma_basic[0];
     fp.extractor = extractor_of(c->prm.extractor_exp);
     fp.precision = c->precision;

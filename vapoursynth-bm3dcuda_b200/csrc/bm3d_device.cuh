@@ -239,18 +239,16 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
 // ---------------------------------------------------------------------------
 // Correctly rounded reciprocal for normal a whose reciprocal is normal
 // (2^-126 <= |a| < 2^126), without a slow-path call: hardware approximation,
-// one Newton-Raphson step, then Markstein's correction y + y * (1 - a * y)
-// with the residual formed exactly by an FMA (P. Markstein, "IA-64 and
-// Elementary Functions", Prentice Hall 2000, ch. 8). Checked bit-exact against
-// the IEEE reciprocal over every float of that range by
-// bm3d_b200_selftest_reciprocal.
+// then Markstein's correction y + y * (1 - a * y) with the residual formed
+// exactly by an FMA (P. Markstein, "IA-64 and Elementary Functions", Prentice
+// Hall 2000, ch. 8). Bit-exact against the IEEE reciprocal over every float of
+// that range (bm3d_b200_selftest_reciprocal); a Newton-Raphson step between the
+// two changes no result.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float rcp_rn_normal(float a) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(a));
-    float e = __fmaf_rn(-a, y, 1.0f);
-    y = __fmaf_rn(e, y, y);
-    e = __fmaf_rn(-a, y, 1.0f);
+    const float e = __fmaf_rn(-a, y, 1.0f);
     return __fmaf_rn(e, y, y);
 }
 

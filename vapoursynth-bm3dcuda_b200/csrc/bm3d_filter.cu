@@ -17,8 +17,11 @@
 // column frequency, in-register index = group frequency * 8 + row frequency),
 // so the Wiener weight's sum of squares is accumulated in the same order.
 //
-// Scatter: the 8 threads of a group add 8 contiguous pixels of a patch row per
-// instruction, so a warp's reduction touches 4-8 sectors instead of 32. With
+// Scatter: where the accumulators lie in one allocation with corner weights
+// (the clip and batch paths; scatter_map has the conditions), each patch goes as
+// one TMA reduction of a 12 x 8 box, which takes the 64 additions per thread off
+// the load/store pipe. Elsewhere (raw stacks, single windows) the 8 threads of a
+// group add 8 contiguous pixels of a patch row per instruction. With
 // corner weights the weight of a patch is added once, at its top-left pixel;
 // the aggregation kernel then sums each pixel's 8x8 neighbourhood of corners,
 // which equals the per-pixel weight sum (exactly so with pre-rounding).
@@ -26,6 +29,16 @@
 // Groups are scheduled block-row-major across windows: CTAs running together
 // work on the same rows of every window, so the gathered patches and the
 // accumulator rows they hit stay resident in L2.
+//
+// Bound: the load/store pipe and the issue slots, then the L2's additions. Of
+// the 30-window 1920x1080 radius-2 launches (hard threshold / Wiener): gathers
+// alone take 0.30 / 0.60 ms, the additions alone 0.57 (as reductions of the
+// load/store pipe) or 0.70 (TMA, in parallel). 1.25 / 2.41 ms before, 1.09 /
+// 1.98 with the scatter by TMA, 0.97 / 1.79 with the paired layout exchanges,
+// 0.99 / 1.73 with packed scatter arithmetic kept exact and the prefetch loop
+// rolled: at 48 KB of code the Wiener kernel's warps waited for instructions
+// (1.4 stalls per issue, 0.44 after).
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -36,35 +49,91 @@ namespace bm3d {
 
 namespace {
 
-constexpr int kXchgGroup = 584;  // words per group in the exchange buffer (8*72 + 8)
-constexpr int kCoefGroup = 520;  // words per group of parked Wiener coefficients
+constexpr int kXchgGroup = 528;    // words per group in the exchange buffer (8*64 + 16)
+constexpr int kXchgGroupTc = 584;  // the split-BF16 form's: rows of 9 words (8*72 + 8)
+constexpr int kCoefGroup = 520;    // words per group of parked Wiener coefficients
 constexpr int kGroupsPerCta = 16;
+// Scatter boxes of the TMA form: a patch's 8 rows of 12 words (the 8 pixels and
+// the words that complete their 16-byte quads), 128-byte aligned.
+constexpr int kBoxWords = 96, kBoxGroup = 8 * kBoxWords;
+
+// Layout exchanges between the 8 threads of a group (thread = column or row of
+// the group's patches), through shared memory. Every access moves 128 bytes per
+// wavefront without bank conflicts; what the two layouts choose is which values
+// arrive in adjacent registers, since the pass that follows works on packed
+// pairs and re-pairing 64 values costs moves:
+//   pairs of patches (p, p + 1), before a pass within the patches
+//     (col_to_row): the pair is one 8-byte unit; unit (row i, column c) of patch
+//     pair q at word q*128 + i*16 + 2c with its 16-byte quads permuted by i / 2:
+//     32 8-byte stores, 16 16-byte loads
+//   pairs of rows (r, r + 1), before a pass across the group (row_to_col): unit
+//     (r / 2, c) of patch p at word p*64 + (r / 2)*16 + 2 (c ^ f), f from r and the
+//     group: 64 single stores, 32 8-byte loads
+// against 64 and 64 single-word accesses each way.
+
+// c ^ this is column c's unit in row pair r2 of group g (pairs-of-rows layout):
+// with the groups 16 words apart, the 32 lanes of a store (8 rows x 4 groups)
+// and the 16 of a load's half warp (8 columns x 2 groups) hit distinct banks.
+__device__ __forceinline__ int row_pair_swizzle(int r2, int g) {
+    return (r2 >> 1) | (g & 2) | ((r2 & 1) << 2);
+}
 
 // thread = column `me`, v[p][row] -> thread = row `me`, v[p][col]
 __device__ __forceinline__ void col_to_row(float (&v)[8][8], float *S, int me) {
 #pragma unroll
-    for (int p = 0; p < 8; ++p)
+    for (int i = 0; i < 8; ++i) {
+        float *unit = S + i * 16 + (((me >> 1) ^ (i >> 1)) << 2) + ((me & 1) << 1);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) S[p * 72 + i * 9 + me] = v[p][i];
+        for (int q = 0; q < 4; ++q)
+            *reinterpret_cast<float2 *>(unit + q * 128) = make_float2(v[2 * q][i], v[2 * q + 1][i]);
+    }
     __syncwarp();
 #pragma unroll
-    for (int p = 0; p < 8; ++p)
+    for (int c = 0; c < 8; c += 2) {
+        const float *quad = S + me * 16 + (((c >> 1) ^ (me >> 1)) << 2);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[p][j] = S[p * 72 + me * 9 + j];
+        for (int q = 0; q < 4; ++q) {
+            const float4 t = *reinterpret_cast<const float4 *>(quad + q * 128);
+            v[2 * q][c] = t.x;
+            v[2 * q + 1][c] = t.y;
+            v[2 * q][c + 1] = t.z;
+            v[2 * q + 1][c + 1] = t.w;
+        }
+    }
     __syncwarp();
 }
 
+// thread = row `me`: v[p][col] into the pairs-of-rows layout of group g
+__device__ __forceinline__ void put_row(float *S, const float (&v)[8][8], int me, int g) {
+    const int f = row_pair_swizzle(me >> 1, g);
+    float *row = S + (me >> 1) * 16 + (me & 1);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        float *unit = row + ((c ^ f) << 1);
+#pragma unroll
+        for (int p = 0; p < 8; ++p) unit[p * 64] = v[p][c];
+    }
+}
+
+// word of (row r, column c) of patch 0 in the pairs-of-rows layout of group g
+__device__ __forceinline__ int row_pair_word(int r, int c, int g) {
+    return (r >> 1) * 16 + ((c ^ row_pair_swizzle(r >> 1, g)) << 1) + (r & 1);
+}
+
 // thread = row `me`, v[p][col] -> thread = column `me`, v[p][row]
-__device__ __forceinline__ void row_to_col(float (&v)[8][8], float *S, int me) {
-#pragma unroll
-    for (int p = 0; p < 8; ++p)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) S[p * 72 + me * 9 + j] = v[p][j];
+__device__ __forceinline__ void row_to_col(float (&v)[8][8], float *S, int me, int g) {
+    put_row(S, v, me, g);
     __syncwarp();
 #pragma unroll
-    for (int p = 0; p < 8; ++p)
+    for (int r = 0; r < 8; r += 2) {
+        const float *unit = S + row_pair_word(r, me, g);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[p][i] = S[p * 72 + i * 9 + me];
+        for (int p = 0; p < 8; ++p) {
+            const float2 t = *reinterpret_cast<const float2 *>(unit + p * 64);
+            v[p][r] = t.x;
+            v[p][r + 1] = t.y;
+        }
+    }
     __syncwarp();
 }
 
@@ -114,21 +183,21 @@ __device__ __forceinline__ void pass_across_group_var(float (&v)[8][8], bool for
     }
 }
 
-__device__ __forceinline__ void forward3d_var(float (&v)[8][8], float *S, int me, int t2d,
+__device__ __forceinline__ void forward3d_var(float (&v)[8][8], float *S, int me, int g, int t2d,
                                               int t1d) {
     pass_in_patch_var(v, true, t2d);
     col_to_row(v, S, me);
     pass_in_patch_var(v, true, t2d);
-    row_to_col(v, S, me);
+    row_to_col(v, S, me, g);
     pass_across_group_var(v, true, t1d);
 }
 
 // Forward 3-D transform: in thread = column layout, out thread = column layout.
-__device__ __forceinline__ void forward3d(float (&v)[8][8], float *S, int me) {
+__device__ __forceinline__ void forward3d(float (&v)[8][8], float *S, int me, int g) {
     pass_in_patch(v, true);   // rows (vertical)
     col_to_row(v, S, me);
     pass_in_patch(v, true);   // columns (horizontal)
-    row_to_col(v, S, me);
+    row_to_col(v, S, me, g);
     pass_across_group(v, true);
 }
 
@@ -198,12 +267,12 @@ __device__ __forceinline__ int tc_addr(int axis, int l, int k) {
                                  : k * 72 + (l >> 3) * 9 + (l & 7);
 }
 
-// One pass along `axis` for the warp's four groups (buffers kXchgGroup apart).
+// One pass along `axis` for the warp's four groups (buffers kXchgGroupTc apart).
 __device__ __forceinline__ void tc_pass(float *W, int axis, const SplitB &B, int lane) {
     const int gq = lane >> 2, t = lane & 3;
 #pragma unroll 1
     for (int gi = 0; gi < 4; ++gi) {
-        float *G = W + gi * kXchgGroup;
+        float *G = W + gi * kXchgGroupTc;
 #pragma unroll
         for (int mt = 0; mt < 4; ++mt) {
             const int l0 = mt * 16 + gq, l1 = l0 + 8;
@@ -258,6 +327,14 @@ __device__ __forceinline__ void tc_transform3d(float (&v)[8][8], float *S, float
     }
 }
 
+// The position of patch `me`.
+__device__ __forceinline__ int pick_pos(const int (&pos)[8], int me) {
+    int q = pos[0];
+#pragma unroll
+    for (int k = 1; k < 8; ++k) q = me == k ? pos[k] : q;
+    return q;
+}
+
 __device__ __forceinline__ void load_group(float (&v)[8][8], const float *const *planes,
                                            const int (&pos)[8], int stride, int c) {
 #pragma unroll
@@ -270,35 +347,159 @@ __device__ __forceinline__ void load_group(float (&v)[8][8], const float *const 
 
 // The same pixels as load_group, copied asynchronously into C[(p*8 + r)*8 + c]
 // (the thread's own slots of the parked-coefficient buffer): they land while
-// the thread works on something else, and only this thread reads them.
-__device__ __forceinline__ void prefetch_group(float *C, const float *const *planes,
-                                               const int (&pos)[8], int stride, int c) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(C + c);
-#pragma unroll
-    for (int p = 0; p < 8; ++p) {
-        const float *b = planes[pos_z(pos[p])] + (size_t)pos_y(pos[p]) * stride + pos_x(pos[p]) + c;
+// the thread works on something else, and only this thread reads them. A rolled
+// loop (patch p's position comes from lane p): the Wiener kernel's code is at
+// the size where warps wait for instructions.
+__device__ __forceinline__ void prefetch_group(float *C, const float *const *planes, int pos_me,
+                                               int stride, int c) {
+    unsigned d = (unsigned)__cvta_generic_to_shared(C + c);
+#pragma unroll 1
+    for (int p = 0; p < 8; ++p, d += 256u) {
+        const int pos = __shfl_sync(0xffffffffu, pos_me, p, 8);
+        const float *b = planes[pos_z(pos)] + (size_t)pos_y(pos) * stride + pos_x(pos) + c;
 #pragma unroll
         for (int r = 0; r < 8; ++r)
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d + 4u * (p * 64 + r * 8)),
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d + 32u * r),
                          "l"(b + (size_t)r * stride)
                          : "memory");
     }
 }
 
-template <bool FINAL>
+// Shared-memory words of a warp: its four groups' exchange buffers, then their
+// parked Wiener coefficients; the scatter boxes of the TMA form take their place.
+template <bool FINAL, bool TC, bool TMA>
+__host__ __device__ constexpr int warp_words() {
+    constexpr int work = 4 * ((TC ? kXchgGroupTc : kXchgGroup) + (FINAL ? kCoefGroup : 0));
+    return TMA && work < 4 * kBoxGroup ? 4 * kBoxGroup : work;
+}
+
+template <bool FINAL, bool TC, bool TMA>
 constexpr size_t filter_smem() {
-    return (size_t)kGroupsPerCta * (kXchgGroup + (FINAL ? kCoefGroup : 0)) * sizeof(float);
+    return (size_t)(kGroupsPerCta / 4) * warp_words<FINAL, TC, TMA>() * sizeof(float);
+}
+
+// Weighted scatter (source/kernel.cu:717-756) by reductions of the load/store
+// pipe, from the exchange buffer.
+template <bool TC>
+__device__ __forceinline__ void scatter_lsu(const FilterParams &prm, const float *S, float weight,
+                                            const int (&pos)[8], int win, bool active, int me,
+                                            int g) {
+    const int tw = 2 * prm.radius + 1;
+    // thread `me` owns column
+    // `me` of every patch and adds one patch per iteration of a rolled loop
+    // (the patch position comes from lane `p` of the group). Pre-rounding with
+    // 2^extractor_exp makes the sums independent of the atomic order; a
+    // multiplicity of 1 multiplies exactly.
+    // Lane `me` resolves patch `me`'s target (plane pointer, multiplicity)
+    // once; the loop takes patch p's from lane p of the group.
+    const int pos_me = pick_pos(pos, me);
+    const int z_me = pos_z(pos_me);
+    float *const plane_me = prm.acc[(size_t)win * tw + z_me];
+    const float mul_me = prm.mult ? prm.mult[(size_t)win * tw + z_me] : 1.0f;
+    const unsigned long long dst_me =
+        plane_me ? reinterpret_cast<unsigned long long>(
+                       plane_me + (size_t)pos_y(pos_me) * prm.acc_stride + pos_x(pos_me))
+                 : 0ull;
+    const float ext = prm.extractor;
+    const float wq = __fsub_rn(__fadd_rn(weight, ext), ext);
+#pragma unroll 1
+    for (int p = 0; p < 8; ++p) {
+        float *wd = reinterpret_cast<float *>(__shfl_sync(0xffffffffu, dst_me, p, 8));
+        const float mul = __shfl_sync(0xffffffffu, mul_me, p, 8);
+        if (!active || wd == nullptr) continue;
+        const float wm = __fmul_rn(wq, mul);
+        float *wt = wd + prm.weight_offset;
+        const float *sp = S + p * (TC ? 72 : 64);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            float val = __fmul_rn(weight, TC ? sp[r * 9 + me] : sp[row_pair_word(r, me, g)]);
+            val = __fsub_rn(__fadd_rn(val, ext), ext);
+            atomicAdd(wd + (size_t)r * prm.acc_stride + me, __fmul_rn(val, mul));
+            if (!prm.corner_weight) atomicAdd(wt + (size_t)r * prm.acc_stride + me, wm);
+        }
+        if (prm.corner_weight && me == 0) atomicAdd(wt, wm);
+    }
+}
+
+// Row `me` of a patch's box: the 8 values at words o .. o + 7 of 12, zeros
+// around them (adding zero leaves a neighbour's sum as it is).
+__device__ __forceinline__ void store_box_row(float *row, const float (&v)[8], int o) {
+    float t[9], u[12];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+        const float same = i < 8 ? v[i < 8 ? i : 0] : 0.0f, left = i > 0 ? v[i > 0 ? i - 1 : 0] : 0.0f;
+        t[i] = o & 1 ? left : same;
+    }
+#pragma unroll
+    for (int i = 0; i < 12; ++i) {
+        const float same = i < 9 ? t[i < 9 ? i : 0] : 0.0f;
+        const float left = i > 1 && i < 11 ? t[i > 1 && i < 11 ? i - 2 : 0] : 0.0f;
+        u[i] = o & 2 ? left : same;
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        *reinterpret_cast<float4 *>(row + 4 * i) =
+            make_float4(u[4 * i], u[4 * i + 1], u[4 * i + 2], u[4 * i + 3]);
+}
+
+// Weighted scatter of a warp's four groups by TMA reductions (thread = row `me`
+// of group g, v[p][column]): each patch goes as one 8 x 12 box added to the
+// accumulators, from the 16-byte boundary at or below its first pixel, so
+// that the additions leave the load/store pipe, which bounds the filter. Lane
+// `me` issues patch `me`'s box. Same terms as scatter_lsu below.
+__device__ __forceinline__ void scatter_tma(const FilterParams &prm, const CUtensorMap *map,
+                                            float *box, const float (&v)[8][8], float weight,
+                                            const int (&pos)[8], int win, bool active, int me) {
+    const int tw = 2 * prm.radius + 1;
+    const int pos_me = pick_pos(pos, me);
+    const int z_me = pos_z(pos_me);
+    float *const plane_me = prm.acc[(size_t)win * tw + z_me];
+    const float mul_me = prm.mult ? prm.mult[(size_t)win * tw + z_me] : 1.0f;
+    const float ext = prm.extractor;
+    const float wq = __fsub_rn(__fadd_rn(weight, ext), ext);
+#pragma unroll
+    for (int p = 0; p < 8; ++p) {
+        const float mul = __shfl_sync(0xffffffffu, mul_me, p, 8);
+        float t[8];
+#pragma unroll
+        for (int j = 0; j < 8; j += 2) {
+            // + ext in scalar form: the assembler contracts a packed product
+            // with a packed sum (seen as 3 of 9600 outputs off by a quantum)
+            float a, b;
+            unpack2(mul2(splat2(weight), pack2(v[p][j], v[p][j + 1])), a, b);
+            const f32x2 sum = pack2(__fadd_rn(a, ext), __fadd_rn(b, ext));
+            unpack2(mul2(sub2(sum, splat2(ext)), splat2(mul)), t[j], t[j + 1]);
+        }
+        store_box_row(box + p * kBoxWords + me * 12, t, pos[p] & 3);
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (active && plane_me != nullptr) {
+        // the target's index among the accumulator pairs, exact below 2^20 pairs
+        const int pair = __float2int_rn((float)(plane_me - prm.acc_base) * prm.acc_pair_inv);
+        const int y = pair * prm.acc_pair_rows + pos_y(pos_me);
+        asm volatile(
+            "cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], "
+            "[%3];" ::"l"(map),
+            "r"(pos_x(pos_me) & ~3), "r"(y),
+            "r"((unsigned)__cvta_generic_to_shared(box + me * kBoxWords))
+            : "memory");
+        atomicAdd(plane_me + prm.weight_offset + (size_t)pos_y(pos_me) * prm.acc_stride +
+                      pos_x(pos_me),
+                  __fmul_rn(wq, mul_me));
+    }
+    // the boxes stay until they have been read
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
 
 // The kGroupsPerCta groups of CTA index `cta` of one filter launch; TC runs
 // the transforms on the tensor cores (split BF16), else in FP32 with the
 // reference's factorisation; VAR takes the transform kinds from prm.t2d /
 // prm.t1d (FP32).
-template <bool FINAL, bool TC, bool VAR = false>
-__device__ __forceinline__ void filter_cta(const FilterParams &prm, long long cta, float *fsm) {
-    float *xbuf = fsm;
-    float *cbuf = fsm + kGroupsPerCta * kXchgGroup;
-
+template <bool FINAL, bool TC, bool VAR, bool TMA>
+__device__ __forceinline__ void filter_cta(const FilterParams &prm, const CUtensorMap *map,
+                                           long long cta, float *fsm) {
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int g = lane >> 3;
@@ -314,8 +515,9 @@ __device__ __forceinline__ void filter_cta(const FilterParams &prm, long long ct
     const int blk = brow * prm.nbx + (int)(rem - (long long)wrel * prm.nbx);
     const int win = prm.win0 + wrel;
     const int tw = 2 * prm.radius + 1;
-    float *S = xbuf + (warp * 4 + g) * kXchgGroup;
-    float *W = xbuf + warp * 4 * kXchgGroup;
+    constexpr int kXchg = TC ? kXchgGroupTc : kXchgGroup;
+    float *W = fsm + warp * warp_words<FINAL, TC, TMA>();
+    float *S = W + g * kXchg;
     SplitB Bf{}, Bi{};
     if (TC) {
         Bf = dct_fragment(true, lane);
@@ -344,8 +546,8 @@ __device__ __forceinline__ void filter_cta(const FilterParams &prm, long long ct
         // its own slots of C: the basic spectrum's Wiener coefficients in,
         // the noisy pixels out, and the noisy group is transformed and
         // scaled by 1/4096 and its coefficient (the reference's two roundings).
-        float *C = cbuf + (warp * 4 + g) * kCoefGroup;
-        prefetch_group(C, prm.src + (size_t)win * tw, pos, prm.stride, me);
+        float *C = W + 4 * kXchg + g * kCoefGroup;
+        prefetch_group(C, prm.src + (size_t)win * tw, pick_pos(pos, me), prm.stride, me);
         load_group(v, prm.ref + (size_t)win * tw, pos, prm.stride, me);
         const float sqr_sigma = __fmul_rn(sigma, sigma);
         float norm = 0.0f;
@@ -354,8 +556,8 @@ __device__ __forceinline__ void filter_cta(const FilterParams &prm, long long ct
 #pragma unroll 1
         for (int it = 0; it < 2; ++it) {
             if (TC) tc_transform3d(v, S, W, me, lane, Bf);
-            else if (VAR) forward3d_var(v, S, me, prm.t2d, prm.t1d);
-            else forward3d(v, S, me);
+            else if (VAR) forward3d_var(v, S, me, g, prm.t2d, prm.t1d);
+            else forward3d(v, S, me, g);
             if (it == 1) break;
             asm volatile("cp.async.wait_all;" ::: "memory");
             // Two coefficients (rows r, r + 1) per packed FP32x2 instruction
@@ -370,11 +572,9 @@ __device__ __forceinline__ void filter_cta(const FilterParams &prm, long long ct
                     const f32x2 x = pack2(v[p][r], v[p][r + 1]);
                     const f32x2 sq = mul2(x, x);
                     // sq + sigma^2 >= sigma^2 >= (FLT_EPSILON * 0.188)^2: a normal float
-                    const f32x2 den = add2(sq, sig2);
+                    const f32x2 den = add2(sq, sig2), nden = mul2(den, splat2(-1.0f));
                     f32x2 y = pack2(rcp_approx(lo2(den)), rcp_approx(hi2(den)));
-                    f32x2 e = fma2(neg2(den), y, one2);  // reciprocal as rcp_rn_normal
-                    y = fma2(e, y, y);
-                    e = fma2(neg2(den), y, one2);
+                    f32x2 e = fma2(nden, y, one2);  // reciprocal as rcp_rn_normal
                     y = fma2(e, y, y);
                     float c0, c1;
                     unpack2(mul2(sq, y), c0, c1);
@@ -392,8 +592,13 @@ __device__ __forceinline__ void filter_cta(const FilterParams &prm, long long ct
 #pragma unroll
         for (int p = 0; p < 8; ++p)
 #pragma unroll
-            for (int r = 0; r < 8; ++r)
-                v[p][r] = __fmul_rn(__fmul_rn(v[p][r], inv4096), C[(p * 8 + r) * 8 + me]);
+            for (int r = 0; r < 8; r += 2) {
+                const float *slot = C + (p * 8 + r) * 8 + me;
+                float x0, x1;
+                unpack2(mul2(pack2(v[p][r], v[p][r + 1]), splat2(inv4096)), x0, x1);
+                v[p][r] = __fmul_rn(x0, slot[0]);
+                v[p][r + 1] = __fmul_rn(x1, slot[8]);
+            }
         norm = __fadd_rn(norm, __shfl_xor_sync(0xffffffffu, norm, 1, 8));
         norm = __fadd_rn(norm, __shfl_xor_sync(0xffffffffu, norm, 2, 8));
         norm = __fadd_rn(norm, __shfl_xor_sync(0xffffffffu, norm, 4, 8));
@@ -402,8 +607,8 @@ __device__ __forceinline__ void filter_cta(const FilterParams &prm, long long ct
         // hard thresholding (source/kernel.cu:208-252, cpu_source/source.cpp:562-594)
         load_group(v, prm.src + (size_t)win * tw, pos, prm.stride, me);
         if (TC) tc_transform3d(v, S, W, me, lane, Bf);
-        else if (VAR) forward3d_var(v, S, me, prm.t2d, prm.t1d);
-        else forward3d(v, S, me);
+        else if (VAR) forward3d_var(v, S, me, g, prm.t2d, prm.t1d);
+        else forward3d(v, S, me, g);
         int nnz = 0;
 #pragma unroll
         for (int p = 0; p < 8; ++p) {
@@ -413,19 +618,30 @@ __device__ __forceinline__ void filter_cta(const FilterParams &prm, long long ct
                 const float x = v[p][r];
                 const bool keep = fabsf(x) >= thr;
                 nnz += keep ? 1 : 0;
-                v[p][r] = keep ? __fmul_rn(x, inv4096) : 0.0f;
+                v[p][r] = keep ? x : 0.0f;
             }
         }
+#pragma unroll
+        for (int p = 0; p < 8; p += 2)
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+                unpack2(mul2(pack2(v[p][r], v[p + 1][r]), splat2(inv4096)), v[p][r], v[p + 1][r]);
         nnz += __shfl_xor_sync(0xffffffffu, nnz, 1, 8);
         nnz += __shfl_xor_sync(0xffffffffu, nnz, 2, 8);
         nnz += __shfl_xor_sync(0xffffffffu, nnz, 4, 8);
         weight = __fdiv_rn(1.0f, (float)nnz);
     }
 
-    // inverse: rows, columns, group; the result is left in the exchange
-    // buffer as S[p*72 + r*9 + c]
+    // inverse: rows, columns, group
     if (TC) {
         tc_transform3d<false>(v, S, W, me, lane, Bi);
+        if constexpr (TMA) {
+#pragma unroll
+            for (int p = 0; p < 8; ++p)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) v[p][j] = S[p * 72 + me * 9 + j];
+            __syncwarp();
+        }
     } else {
         if (VAR) {
             pass_in_patch_var(v, false, prm.t2d);
@@ -438,71 +654,40 @@ __device__ __forceinline__ void filter_cta(const FilterParams &prm, long long ct
             pass_in_patch(v, false);
             pass_across_group(v, false);
         }
-#pragma unroll
-        for (int p = 0; p < 8; ++p)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) S[p * 72 + me * 9 + j] = v[p][j];
-        __syncwarp();
-    }
-
-    // weighted scatter (source/kernel.cu:717-756); thread `me` owns column
-    // `me` of every patch and adds one patch per iteration of a rolled loop
-    // (the patch position comes from lane `p` of the group). Pre-rounding with
-    // 2^extractor_exp makes the sums independent of the atomic order; a
-    // multiplicity of 1 multiplies exactly.
-    // Lane `me` resolves patch `me`'s target (plane pointer, multiplicity)
-    // once; the loop takes patch p's from lane p of the group.
-    int pos_me = pos[0];
-#pragma unroll
-    for (int k = 1; k < 8; ++k) pos_me = me == k ? pos[k] : pos_me;
-    const int z_me = pos_z(pos_me);
-    float *const plane_me = prm.acc[(size_t)win * tw + z_me];
-    const float mul_me = prm.mult ? prm.mult[(size_t)win * tw + z_me] : 1.0f;
-    const unsigned long long dst_me =
-        plane_me ? reinterpret_cast<unsigned long long>(
-                       plane_me + (size_t)pos_y(pos_me) * prm.acc_stride + pos_x(pos_me))
-                 : 0ull;
-    const float ext = prm.extractor;
-    const float wq = __fsub_rn(__fadd_rn(weight, ext), ext);
-#pragma unroll 1
-    for (int p = 0; p < 8; ++p) {
-        float *wd = reinterpret_cast<float *>(__shfl_sync(0xffffffffu, dst_me, p, 8));
-        const float mul = __shfl_sync(0xffffffffu, mul_me, p, 8);
-        if (!active || wd == nullptr) continue;
-        const float wm = __fmul_rn(wq, mul);
-        float *wt = wd + prm.weight_offset;
-        const float *sp = S + p * 72 + me;
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            float val = __fmul_rn(weight, sp[r * 9]);
-            val = __fsub_rn(__fadd_rn(val, ext), ext);
-            atomicAdd(wd + (size_t)r * prm.acc_stride + me, __fmul_rn(val, mul));
-            if (!prm.corner_weight) atomicAdd(wt + (size_t)r * prm.acc_stride + me, wm);
+        if constexpr (!TMA) {
+            put_row(S, v, me, g);
+            __syncwarp();
         }
-        if (prm.corner_weight && me == 0) atomicAdd(wt, wm);
     }
+    if constexpr (TMA)
+        scatter_tma(prm, map, W + g * kBoxGroup, v, weight, pos, win, active, me);
+    else
+        scatter_lsu<TC>(prm, S, weight, pos, win, active, me, g);
 }
+
 
 // Resident CTAs per SM the register allocation aims at: the hard-threshold
 // FP32 kernel fits 96 registers without spills (5 CTAs: 1.30 ms against 1.33
-// at 4 for the 30-window launch); the Wiener kernel's shared memory allows 3.
-template <bool FINAL, bool TC, bool VAR>
+// at 4 for the 30-window launch), its TMA form's boxes allow 4; the Wiener
+// kernel's shared memory allows 3.
+template <bool FINAL, bool TC, bool VAR, bool TMA>
 constexpr int filter_ctas_per_sm() {
-    return FINAL ? 3 : (TC || VAR ? 4 : 5);
+    return FINAL ? 3 : (TC || VAR || TMA ? 4 : 5);
 }
 
-template <bool FINAL, bool TC, bool VAR = false>
-__global__ void __launch_bounds__(128, filter_ctas_per_sm<FINAL, TC, VAR>())
-    filter_kernel(FilterParams prm) {
-    extern __shared__ float fsm[];
-    filter_cta<FINAL, TC, VAR>(prm, blockIdx.x, fsm);
+template <bool FINAL, bool TC, bool VAR, bool TMA>
+__global__ void __launch_bounds__(128, filter_ctas_per_sm<FINAL, TC, VAR, TMA>())
+    filter_kernel(FilterParams prm, const __grid_constant__ CUtensorMap map) {
+    extern __shared__ __align__(128) float fsm[];
+    filter_cta<FINAL, TC, VAR, TMA>(prm, &map, blockIdx.x, fsm);
 }
 
 // Persistent form over a batch of clips: resident CTAs take CTA-sized group
-// ranges from a shared counter, clip-major.
-template <bool FINAL>
-__global__ void __launch_bounds__(128, 3) filter_batch_kernel(FilterBatch b) {
-    extern __shared__ float fsm[];
+// ranges from a shared counter, clip-major. TMA: every clip has a tensor map.
+template <bool FINAL, bool TMA>
+__global__ void __launch_bounds__(128, filter_ctas_per_sm<FINAL, false, false, true>())
+    filter_batch_kernel(FilterBatch b) {
+    extern __shared__ __align__(128) float fsm[];
     __shared__ FilterParams ps;
     __shared__ long long item_s;
     const long long total = b.item_off[b.nclips];
@@ -518,7 +703,8 @@ __global__ void __launch_bounds__(128, 3) filter_batch_kernel(FilterBatch b) {
         }
         if (threadIdx.x == 0) ps = b.clips[lo];
         __syncthreads();
-        filter_cta<FINAL, false>(ps, item - b.item_off[lo], fsm);
+        filter_cta<FINAL, false, false, TMA>(ps, TMA ? b.maps + lo : nullptr,
+                                             item - b.item_off[lo], fsm);
         __syncthreads();
     }
 }
@@ -697,18 +883,61 @@ __global__ void vaggregate_kernel(VAggregateParams p) {
 
 namespace {
 
-template <bool FINAL, bool TC, bool VAR = false>
-cudaError_t launch_filter_t(const FilterParams &p, dim3 grid, cudaStream_t stream) {
+template <bool FINAL, bool TC, bool VAR, bool TMA>
+cudaError_t launch_filter_t(const FilterParams &p, const CUtensorMap &map, dim3 grid,
+                            cudaStream_t stream) {
     // opt in to more than 48 KB of dynamic shared memory once per device
     static int configured[64] = {};
-    cudaError_t e = raise_smem_limit(configured, (const void *)filter_kernel<FINAL, TC, VAR>,
-                                      filter_smem<FINAL>());
+    const auto fn = filter_kernel<FINAL, TC, VAR, TMA>;
+    constexpr size_t smem = filter_smem<FINAL, TC, TMA>();
+    cudaError_t e = raise_smem_limit(configured, (const void *)fn, smem);
     if (e != cudaSuccess) return e;
-    filter_kernel<FINAL, TC, VAR><<<grid, 128, filter_smem<FINAL>(), stream>>>(p);
+    fn<<<grid, 128, smem, stream>>>(p, map);
     return cudaGetLastError();
 }
 
+template <bool TC, bool VAR>
+cudaError_t launch_filter_form(const FilterParams &p, bool final_, dim3 grid,
+                               cudaStream_t stream) {
+    CUtensorMap map{};
+    if (scatter_map(p, &map))
+        return final_ ? launch_filter_t<true, TC, VAR, true>(p, map, grid, stream)
+                      : launch_filter_t<false, TC, VAR, true>(p, map, grid, stream);
+    return final_ ? launch_filter_t<true, TC, VAR, false>(p, map, grid, stream)
+                  : launch_filter_t<false, TC, VAR, false>(p, map, grid, stream);
+}
+
 }  // namespace
+
+bool scatter_map(const FilterParams &p, CUtensorMap *map) {
+    using Encode = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
+                                const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
+                                const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static const Encode encode = [] {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found) !=
+                cudaSuccess ||
+            found != cudaDriverEntryPointSuccess)
+            fn = nullptr;
+        return reinterpret_cast<Encode>(fn);
+    }();
+    // the box starts on a 16-byte boundary of its row; pair indices are exact
+    // below 2^20, and rows are 32-bit coordinates
+    if (!encode || !p.corner_weight || !p.acc_base || p.acc_stride % 4 != 0 ||
+        reinterpret_cast<unsigned long long>(p.acc_base) % 16 != 0 || p.acc_pairs >= (1 << 20) ||
+        (long long)p.acc_pairs * p.acc_pair_rows > 0x7fffffffLL)
+        return false;
+    const cuuint64_t dims[2] = {(cuuint64_t)p.acc_stride,
+                                (cuuint64_t)p.acc_pairs * (cuuint64_t)p.acc_pair_rows};
+    const cuuint64_t pitch[1] = {(cuuint64_t)p.acc_stride * sizeof(float)};
+    const cuuint32_t box[2] = {12, 8}, step[2] = {1, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, p.acc_base, dims, pitch, box, step,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                  CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 
 cudaError_t launch_filter(const FilterParams &p, bool final_, cudaStream_t stream) {
     const long long ngroups = (long long)p.nwin * p.nblk;
@@ -720,15 +949,11 @@ cudaError_t launch_filter(const FilterParams &p, bool final_, cudaStream_t strea
     if (p.t2d < 0 || p.t2d > 3 || p.t1d < 0 || p.t1d > 3) return cudaErrorInvalidValue;
     if (p.t2d != 0 || p.t1d != 0) {
         if (p.precision != 0) return cudaErrorInvalidValue;  // variants run in FP32
-        return final_ ? launch_filter_t<true, false, true>(p, grid, stream)
-                      : launch_filter_t<false, false, true>(p, grid, stream);
+        return launch_filter_form<false, true>(p, final_, grid, stream);
     }
     if (p.precision == 2) return launch_filter_tc(p, final_, stream);
-    if (p.precision == 1)
-        return final_ ? launch_filter_t<true, true>(p, grid, stream)
-                      : launch_filter_t<false, true>(p, grid, stream);
-    return final_ ? launch_filter_t<true, false>(p, grid, stream)
-                  : launch_filter_t<false, false>(p, grid, stream);
+    return p.precision == 1 ? launch_filter_form<true, false>(p, final_, grid, stream)
+                            : launch_filter_form<false, false>(p, final_, grid, stream);
 }
 
 namespace {
@@ -747,25 +972,28 @@ int persistent_grid(const void *fn, int threads, size_t smem, int per_sm_want = 
 
 }  // namespace
 
+namespace {
+
+template <bool FINAL, bool TMA>
+cudaError_t launch_filter_batch_t(const FilterBatch &b, cudaStream_t stream, int ctas_per_sm) {
+    static int configured[64] = {};
+    const auto fn = filter_batch_kernel<FINAL, TMA>;
+    constexpr size_t smem = filter_smem<FINAL, false, TMA>();
+    cudaError_t e = raise_smem_limit(configured, (const void *)fn, smem);
+    if (e != cudaSuccess) return e;
+    fn<<<persistent_grid((const void *)fn, 128, smem, ctas_per_sm), 128, smem, stream>>>(b);
+    return cudaGetLastError();
+}
+
+}  // namespace
+
 cudaError_t launch_filter_batch(const FilterBatch &b, bool final_, cudaStream_t stream,
                                 int ctas_per_sm) {
-    static int configured[2][64] = {};
-    cudaError_t e = final_ ? raise_smem_limit(configured[1], (const void *)filter_batch_kernel<true>,
-                                              filter_smem<true>())
-                           : raise_smem_limit(configured[0],
-                                              (const void *)filter_batch_kernel<false>,
-                                              filter_smem<false>());
-    if (e != cudaSuccess) return e;
-    if (final_) {
-        const int grid = persistent_grid((const void *)filter_batch_kernel<true>, 128,
-                                         filter_smem<true>(), ctas_per_sm);
-        filter_batch_kernel<true><<<grid, 128, filter_smem<true>(), stream>>>(b);
-    } else {
-        const int grid = persistent_grid((const void *)filter_batch_kernel<false>, 128,
-                                         filter_smem<false>(), ctas_per_sm);
-        filter_batch_kernel<false><<<grid, 128, filter_smem<false>(), stream>>>(b);
-    }
-    return cudaGetLastError();
+    if (b.maps)
+        return final_ ? launch_filter_batch_t<true, true>(b, stream, ctas_per_sm)
+                      : launch_filter_batch_t<false, true>(b, stream, ctas_per_sm);
+    return final_ ? launch_filter_batch_t<true, false>(b, stream, ctas_per_sm)
+                  : launch_filter_batch_t<false, false>(b, stream, ctas_per_sm);
 }
 
 long long filter_ctas(const FilterParams &p) {

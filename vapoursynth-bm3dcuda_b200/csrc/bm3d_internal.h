@@ -1,6 +1,7 @@
 // Internal launch interfaces of the BM3D kernels (not part of the C ABI).
 #pragma once
 
+#include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -168,10 +169,27 @@ struct FilterParams {
     int precision;      // 0: FP32, the reference's factorisation; 1: split-BF16 tensor
                         // cores; 2: FP16 Kronecker-form 2-D transforms on tcgen05
     int t2d, t1d;       // transforms (rows/columns, group): 0 DCT, 1 Haar, 2 WHT, 3 bior1.5
+    // The targets of `acc` when they all lie in one allocation as acc_pairs pairs
+    // of a wdst and a weight plane (acc_pair_rows rows of acc_stride floats
+    // together), or a null acc_base: what the scatter by TMA needs.
+    float *acc_base;
+    int acc_pairs, acc_pair_rows;
+    float acc_pair_inv;  // 1 / (acc_pair_rows * acc_stride)
     unsigned *err;      // precision 2: set to nonzero when a CTA gave up waiting for its MMAs
 };
 
+// Sets the fields that describe the accumulator pairs (rows: of one plane).
+inline void set_acc_pairs(FilterParams &p, float *base, int pairs, int rows) {
+    p.acc_base = base;
+    p.acc_pairs = pairs;
+    p.acc_pair_rows = 2 * rows;
+    p.acc_pair_inv = 1.0f / ((float)p.acc_pair_rows * (float)p.acc_stride);
+}
+
 cudaError_t launch_filter(const FilterParams &p, bool final_, cudaStream_t stream);
+// The tensor map of the accumulators for the scatter by TMA; false where the
+// launch cannot use it.
+bool scatter_map(const FilterParams &p, CUtensorMap *map);
 // precision 2 (bm3d_filter_tc.cu)
 cudaError_t launch_filter_tc(const FilterParams &p, bool final_, cudaStream_t stream);
 
@@ -195,6 +213,7 @@ struct FilterBatch {
     const long long *item_off;    // [nclips + 1] prefix sums of CTA group ranges
     int nclips;
     unsigned long long *counter;  // zero at launch
+    const CUtensorMap *maps;      // [nclips] scatter_map of each clip (device), or null
 };
 struct AggregateBatch {
     const AggregateParams *clips;  // [nclips] (device); vec precomputed per clip
