@@ -46,3 +46,20 @@ def test_lists_of_every_strip_width(cuda, engine_lib, oracle, bm_range, ps_range
     _, got = graph_run(win, return_matches=True, **kw)
     _, want = oracle.port_bm3d(win, return_matches=True, **kw)
     np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("metric", [1, 2, 3, 4])
+@pytest.mark.parametrize("h,w,step,bm_range,radius,ps_num,ps_range", [
+    (8, 8, 8, 9, 0, 2, 4),       # one block
+    (41, 67, 8, 9, 1, 2, 4),     # strips of 10: 19 and 9 columns
+    (40, 52, 5, 3, 1, 3, 3),     # strips of 8: 7 columns
+    (163, 203, 1, 4, 0, 2, 4),   # one lane per block
+])
+def test_lists_of_other_distances(cuda, engine_lib, oracle, metric, h, w, step, bm_range, radius,
+                                  ps_num, ps_range):
+    win = window(h, w, radius, "texture", seed=metric)
+    kw = dict(sigma=8.0, block_step=step, bm_range=bm_range, radius=radius, ps_num=ps_num,
+              ps_range=ps_range, bm_error=metric)
+    _, got = graph_run(win, return_matches=True, **kw)
+    _, want = oracle.port_bm3d(win, return_matches=True, **kw)
+    np.testing.assert_array_equal(got, want)

@@ -98,6 +98,9 @@ cudaError_t launch_match_split(const MatchParams &p, const MatchGeometry &g, int
                                cudaStream_t stream);
 cudaError_t launch_match_pairs(const MatchParams &p, const MatchGeometry &g, int nwin, int lanes,
                                cudaStream_t stream);
+// launch_match for p.metric != 0, in strips of K (8, 10), with 1 or 4 lanes per block.
+cudaError_t launch_match_metric(const MatchParams &p, const MatchGeometry &g, int nwin, int K,
+                                int lanes, cudaStream_t stream);
 
 // Learned block matching (bm3d_learned.cu): candidate cells ranked by the
 // proposer's embeddings, the best ones scored exactly; blocks whose best

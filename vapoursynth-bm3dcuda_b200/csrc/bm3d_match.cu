@@ -206,27 +206,17 @@ cudaError_t launch_match_split(const MatchParams &p, const MatchGeometry &g, int
 
 cudaError_t launch_match(const MatchParams &p, const MatchGeometry &g, int nwin,
                          cudaStream_t stream) {
+    const int lanes = match_lanes(p, g, nwin);
     if (p.metric != 0) {
-        if (g.smem > kMatchSmemMax) return cudaErrorInvalidValue;
-        dim3 block(32 * g.wx);
-        dim3 grid((p.nbx + 4 * g.wx - 1) / (4 * g.wx), (p.nby + 7) / 8, nwin);
-        // one candidate per strip: the tile (sized for the SSD strips) covers it
-        MatchParams q = p;
-        q.nsub_s = 2 * p.bm_range + 1;
-        q.nsub_t = 2 * p.ps_range + 1;
-        switch (p.metric + (g.small ? 0 : 4)) {
-            case 1: return launch_match_t<1, 1, 1, 1, true>(q, grid, block, g.smem, stream);
-            case 2: return launch_match_t<1, 1, 2, 1, true>(q, grid, block, g.smem, stream);
-            case 3: return launch_match_t<1, 1, 3, 1, true>(q, grid, block, g.smem, stream);
-            case 4: return launch_match_t<1, 1, 4, 1, true>(q, grid, block, g.smem, stream);
-            case 5: return launch_match_t<1, 1, 1, 1, false>(q, grid, block, g.smem, stream);
-            case 6: return launch_match_t<1, 1, 2, 1, false>(q, grid, block, g.smem, stream);
-            case 7: return launch_match_t<1, 1, 3, 1, false>(q, grid, block, g.smem, stream);
-            case 8: return launch_match_t<1, 1, 4, 1, false>(q, grid, block, g.smem, stream);
-            default: return cudaErrorInvalidValue;
-        }
+        const int ws = 2 * p.bm_range + 1, wt = 2 * p.ps_range + 1;
+        const double spatial = (double)ws * ws, temporal = 2.0 * p.radius * p.ps_num * wt * wt;
+        auto cost = [&](int K) {
+            return spatial * strip_cost(ws, K) + temporal * strip_cost(wt, K);
+        };
+        return launch_match_metric(p, g, nwin, cost(10) < cost(8) ? 10 : 8, lanes == 1 ? 1 : 4,
+                                   stream);
     }
-    return launch_match_split(p, g, nwin, match_lanes(p, g, nwin), stream);
+    return launch_match_split(p, g, nwin, lanes, stream);
 }
 
 }  // namespace bm3d

@@ -124,8 +124,7 @@ __device__ __forceinline__ void scan_window(List8 &list, ColumnList &cl, int n,
             if (M == 0) {
                 ssd_strip<K>(refp, tile, roff, err);
             } else {
-#pragma unroll
-                for (int k = 0; k < K; ++k) err[k] = metric_dist<M>(refp, rs, tile, roff, k);
+                metric_strip<K, M>(refp, rs, tile, roff, err);
             }
 #pragma unroll
             for (int r = 0; r < 8; ++r) roff[r] += K;

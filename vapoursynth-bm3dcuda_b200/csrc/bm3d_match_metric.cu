@@ -1,0 +1,56 @@
+// The general matching kernel with the run-time-compiled plugin's distances
+// (bm3d_match_kernels.cuh).
+#include "bm3d_match_kernels.cuh"
+
+namespace bm3d {
+
+namespace {
+
+template <int K, int M, bool SMALL>
+cudaError_t launch_metric(MatchParams q, const MatchGeometry &g, int nwin, int lanes,
+                          cudaStream_t stream) {
+    q.nsub_s = (2 * q.bm_range + K) / K;
+    q.nsub_t = (2 * q.ps_range + K) / K;
+    const int over_s = q.nsub_s * K - (2 * q.bm_range + 1);
+    const int over_t = q.radius > 0 ? q.nsub_t * K - (2 * q.ps_range + 1) : 0;
+    q.extra_cols = std::max(over_s, over_t);
+    const int mmax = q.bm_range + q.radius * q.ps_range;
+    const int wx = lanes == 1 ? g.wx : kSplitWx, wy = lanes == 1 ? 1 : kSplitWy;
+    const int rows = 8 / lanes * wy;  // block rows of a CTA
+    q.pitch = (4 * wx - 1) * q.block_step + 2 * mmax + 16 + q.extra_cols;
+    q.tile_rows = (rows - 1) * q.block_step + 2 * mmax + 8;
+    const size_t smem = (size_t)q.pitch * q.tile_rows * sizeof(float) +
+                        (size_t)(SMALL ? 16 : 8) * 32 * wx * wy * sizeof(int);
+    // a range that only just fits: one candidate per strip needs no extra columns
+    if (smem > kMatchSmemMax)
+        return K == 1 ? cudaErrorInvalidValue
+                      : launch_metric<1, M, false>(q, g, nwin, 1, stream);
+    const dim3 grid((q.nbx + 4 * wx - 1) / (4 * wx), (q.nby + rows - 1) / rows, nwin);
+    const dim3 block(32 * wx * wy);
+    if constexpr (SMALL)
+        if (lanes > 1) return launch_match_t<K, K, M, 4, true>(q, grid, block, smem, stream);
+    return launch_match_t<K, K, M, 1, SMALL>(q, grid, block, smem, stream);
+}
+
+template <int M>
+cudaError_t launch_metric_m(const MatchParams &p, const MatchGeometry &g, int nwin, int K,
+                            int lanes, cudaStream_t stream) {
+    if (p.radius > 0 && p.ps_num > 2) return launch_metric<8, M, false>(p, g, nwin, 1, stream);
+    return K == 10 ? launch_metric<10, M, true>(p, g, nwin, lanes, stream)
+                   : launch_metric<8, M, true>(p, g, nwin, lanes, stream);
+}
+
+}  // namespace
+
+cudaError_t launch_match_metric(const MatchParams &p, const MatchGeometry &g, int nwin, int K,
+                                int lanes, cudaStream_t stream) {
+    switch (p.metric) {
+        case 1: return launch_metric_m<1>(p, g, nwin, K, lanes, stream);
+        case 2: return launch_metric_m<2>(p, g, nwin, K, lanes, stream);
+        case 3: return launch_metric_m<3>(p, g, nwin, K, lanes, stream);
+        case 4: return launch_metric_m<4>(p, g, nwin, K, lanes, stream);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+}  // namespace bm3d
