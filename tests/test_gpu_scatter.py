@@ -41,3 +41,20 @@ def test_reciprocal_is_correctly_rounded(cuda, engine_lib):
     assert engine_lib.bm3d_b200_selftest_reciprocal(0x00800000, 0x7E800000, ctypes.byref(bad),
                                                     ctypes.byref(first)) == 0
     assert bad.value == 0, hex(first.value)
+
+
+@pytest.mark.parametrize("final", [False, True])
+@pytest.mark.parametrize("radius,planes", [(0, 1), (1, 1), (1, 3)])
+@pytest.mark.parametrize("h,w", [(8, 8), (9, 11), (17, 32), (40, 33), (24, 97)])
+def test_weight_boxes_of_a_window(cuda, engine_lib, oracle, h, w, radius, planes, final):
+    """Single windows add a weight to every pixel: both slabs of every slot."""
+    from bm3dcuda import synthetic as S
+    tw = 2 * radius + 1
+    noisy, clean = S.chroma_clip(tw, h, w, seed=w + h)
+    win = noisy[:, :planes].transpose(1, 0, 2, 3).copy()
+    ref = clean[:, :planes].astype(np.float32).transpose(1, 0, 2, 3).copy() if final else None
+    kw = dict(sigma=[7.0, 4.0, 4.0], radius=radius, block_step=3, bm_range=5, extractor_exp=6,
+              chroma=planes == 3)
+    got = graph_run(win, ref, **kw)
+    want = oracle.port_bm3d(win, ref, return_acc=True, **kw)
+    np.testing.assert_array_equal(got, want)

@@ -191,6 +191,7 @@ int graph_enqueue(bm3d_b200_graph *g, cudaStream_t s, bool copies) {
         fp.nblk = g->geo.nbx * g->geo.nby;
         fp.nbx = g->geo.nbx;
         fp.corner_weight = 0;
+        set_acc_pairs(fp, g->d_res, g->nplanes * tw, g->height);
         fp.nwin = 1;
         fp.sigma = g->sigma[q];
         fp.extractor = g->extractor;
@@ -743,7 +744,10 @@ int clip_run_impl(bm3d_b200_clip *c, const float *d_src, const float *d_ref, flo
             fp.nblk = g.nbx * g.nby;
             fp.nbx = g.nbx;
             fp.corner_weight = raw ? 0 : 1;
-            if (!raw) set_acc_pairs(fp, c->d_acc, N, Hq);
+            if (raw)
+                set_raw_pairs(fp, d_dst, N, c->raw_frame_floats, c->rawoff[q], Hq);
+            else
+                set_acc_pairs(fp, c->d_acc, N, Hq);
             fp.nwin = N;
             fp.sigma = sigma;
             fp.extractor = extractor_of(c->prm.extractor_exp);
@@ -1668,6 +1672,7 @@ extern "C" int bm3d_b200_window_noalloc(float *d_res, const float *d_src, int wi
         fp.nblk = (int)nblk;
         fp.nbx = geo.nbx;
         fp.corner_weight = 0;
+        set_acc_pairs(fp, d_res, np * tw, height);
         fp.nwin = 1;
         fp.sigma = sig[q];
         fp.extractor = extractor;
@@ -2108,6 +2113,8 @@ int stream_filter(bm3d_b200_stream *s, bm3d_b200_stream::Request &q,
             fp.nblk = s->geo[mq].nbx * s->geo[mq].nby;
             fp.nbx = s->geo[mq].nbx;
             fp.corner_weight = 0;
+            set_raw_pairs(fp, s->d_raw, (long long)s->wslot.size(), s->raw_floats, s->rawoff[qq],
+                          s->ph[qq]);
             fp.win0 = 0;
             fp.nwin = k;
             fp.sigma = s->sigma[qq];

@@ -56,6 +56,9 @@ constexpr int kGroupsPerCta = 16;
 // Scatter boxes of the TMA form: a patch's 8 rows of 12 words (the 8 pixels and
 // the words that complete their 16-byte quads), 128-byte aligned.
 constexpr int kBoxWords = 96, kBoxGroup = 8 * kBoxWords;
+// Scatter forms: reductions of the load/store pipe; TMA boxes with corner
+// weights; TMA boxes with a weight for every pixel (raw stacks, single windows).
+enum Scatter { kScatterLsu = 0, kScatterBoxes = 1, kScatterWeights = 2 };
 
 // Layout exchanges between the 8 threads of a group (thread = column or row of
 // the group's patches), through shared memory. Every access moves 128 bytes per
@@ -367,15 +370,18 @@ __device__ __forceinline__ void prefetch_group(float *C, const float *const *pla
 
 // Shared-memory words of a warp: its four groups' exchange buffers, then their
 // parked Wiener coefficients; the scatter boxes of the TMA form take their place.
-template <bool FINAL, bool TC, bool TMA>
+template <bool FINAL, bool TC, int SC>
 __host__ __device__ constexpr int warp_words() {
     constexpr int work = 4 * ((TC ? kXchgGroupTc : kXchgGroup) + (FINAL ? kCoefGroup : 0));
-    return TMA && work < 4 * kBoxGroup ? 4 * kBoxGroup : work;
+    constexpr int boxes = 4 * (SC == kScatterLsu       ? 0
+                               : SC == kScatterWeights ? kBoxGroup + 4 * kBoxWords
+                                                       : kBoxGroup);
+    return ((work > boxes ? work : boxes) + 31) / 32 * 32;
 }
 
-template <bool FINAL, bool TC, bool TMA>
+template <bool FINAL, bool TC, int SC>
 constexpr size_t filter_smem() {
-    return (size_t)(kGroupsPerCta / 4) * warp_words<FINAL, TC, TMA>() * sizeof(float);
+    return (size_t)(kGroupsPerCta / 4) * warp_words<FINAL, TC, SC>() * sizeof(float);
 }
 
 // Weighted scatter (source/kernel.cu:717-756) by reductions of the load/store
@@ -446,7 +452,19 @@ __device__ __forceinline__ void store_box_row(float *row, const float (&v)[8], i
 // of group g, v[p][column]): each patch goes as one 8 x 12 box added to the
 // accumulators, from the 16-byte boundary at or below its first pixel, so
 // that the additions leave the load/store pipe, which bounds the filter. Lane
-// `me` issues patch `me`'s box. Same terms as scatter_lsu below.
+// `me` issues patch `me`'s box. Same terms as scatter_lsu.
+// WEIGHTS: the patch's weight goes to all its pixels, as a second box from the
+// one of four (one per column offset) that the group fills with its weight;
+// multiplicities are 1. Else once, at the patch's corner.
+__device__ __forceinline__ void reduce_box(const CUtensorMap *map, int x, int y, const float *box) {
+    asm volatile(
+        "cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], "
+        "[%3];" ::"l"(map),
+        "r"(x), "r"(y), "r"((unsigned)__cvta_generic_to_shared(box))
+        : "memory");
+}
+
+template <bool WEIGHTS>
 __device__ __forceinline__ void scatter_tma(const FilterParams &prm, const CUtensorMap *map,
                                             float *box, const float (&v)[8][8], float weight,
                                             const int (&pos)[8], int win, bool active, int me) {
@@ -472,21 +490,26 @@ __device__ __forceinline__ void scatter_tma(const FilterParams &prm, const CUten
         }
         store_box_row(box + p * kBoxWords + me * 12, t, pos[p] & 3);
     }
+    if constexpr (WEIGHTS) {
+        const float t[8] = {wq, wq, wq, wq, wq, wq, wq, wq};
+#pragma unroll
+        for (int o = 0; o < 4; ++o) store_box_row(box + kBoxGroup + o * kBoxWords + me * 12, t, o);
+    }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();
     if (active && plane_me != nullptr) {
         // the target's index among the accumulator pairs, exact below 2^20 pairs
         const int pair = __float2int_rn((float)(plane_me - prm.acc_base) * prm.acc_pair_inv);
         const int y = pair * prm.acc_pair_rows + pos_y(pos_me);
-        asm volatile(
-            "cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], "
-            "[%3];" ::"l"(map),
-            "r"(pos_x(pos_me) & ~3), "r"(y),
-            "r"((unsigned)__cvta_generic_to_shared(box + me * kBoxWords))
-            : "memory");
-        atomicAdd(plane_me + prm.weight_offset + (size_t)pos_y(pos_me) * prm.acc_stride +
-                      pos_x(pos_me),
-                  __fmul_rn(wq, mul_me));
+        const int x = pos_x(pos_me) & ~3;
+        reduce_box(map, x, y, box + me * kBoxWords);
+        if constexpr (WEIGHTS)
+            reduce_box(map, x, y + (prm.acc_pair_rows >> 1),
+                       box + kBoxGroup + (pos_x(pos_me) & 3) * kBoxWords);
+        else
+            atomicAdd(plane_me + prm.weight_offset + (size_t)pos_y(pos_me) * prm.acc_stride +
+                          pos_x(pos_me),
+                      __fmul_rn(wq, mul_me));
     }
     // the boxes stay until they have been read
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
@@ -497,7 +520,7 @@ __device__ __forceinline__ void scatter_tma(const FilterParams &prm, const CUten
 // the transforms on the tensor cores (split BF16), else in FP32 with the
 // reference's factorisation; VAR takes the transform kinds from prm.t2d /
 // prm.t1d (FP32).
-template <bool FINAL, bool TC, bool VAR, bool TMA>
+template <bool FINAL, bool TC, bool VAR, int SC>
 __device__ __forceinline__ void filter_cta(const FilterParams &prm, const CUtensorMap *map,
                                            long long cta, float *fsm) {
     const int lane = threadIdx.x & 31;
@@ -516,7 +539,7 @@ __device__ __forceinline__ void filter_cta(const FilterParams &prm, const CUtens
     const int win = prm.win0 + wrel;
     const int tw = 2 * prm.radius + 1;
     constexpr int kXchg = TC ? kXchgGroupTc : kXchgGroup;
-    float *W = fsm + warp * warp_words<FINAL, TC, TMA>();
+    float *W = fsm + warp * warp_words<FINAL, TC, SC>();
     float *S = W + g * kXchg;
     SplitB Bf{}, Bi{};
     if (TC) {
@@ -635,7 +658,7 @@ __device__ __forceinline__ void filter_cta(const FilterParams &prm, const CUtens
     // inverse: rows, columns, group
     if (TC) {
         tc_transform3d<false>(v, S, W, me, lane, Bi);
-        if constexpr (TMA) {
+        if constexpr (SC != kScatterLsu) {
 #pragma unroll
             for (int p = 0; p < 8; ++p)
 #pragma unroll
@@ -654,13 +677,16 @@ __device__ __forceinline__ void filter_cta(const FilterParams &prm, const CUtens
             pass_in_patch(v, false);
             pass_across_group(v, false);
         }
-        if constexpr (!TMA) {
+        if constexpr (SC == kScatterLsu) {
             put_row(S, v, me, g);
             __syncwarp();
         }
     }
-    if constexpr (TMA)
-        scatter_tma(prm, map, W + g * kBoxGroup, v, weight, pos, win, active, me);
+    if constexpr (SC == kScatterWeights)
+        scatter_tma<true>(prm, map, W + g * (kBoxGroup + 4 * kBoxWords), v, weight, pos, win,
+                          active, me);
+    else if constexpr (SC == kScatterBoxes)
+        scatter_tma<false>(prm, map, W + g * kBoxGroup, v, weight, pos, win, active, me);
     else
         scatter_lsu<TC>(prm, S, weight, pos, win, active, me, g);
 }
@@ -670,22 +696,22 @@ __device__ __forceinline__ void filter_cta(const FilterParams &prm, const CUtens
 // FP32 kernel fits 96 registers without spills (5 CTAs: 1.30 ms against 1.33
 // at 4 for the 30-window launch), its TMA form's boxes allow 4; the Wiener
 // kernel's shared memory allows 3.
-template <bool FINAL, bool TC, bool VAR, bool TMA>
+template <bool FINAL, bool TC, bool VAR, int SC>
 constexpr int filter_ctas_per_sm() {
-    return FINAL ? 3 : (TC || VAR || TMA ? 4 : 5);
+    return FINAL || SC == kScatterWeights ? 3 : (TC || VAR || SC == kScatterBoxes ? 4 : 5);
 }
 
-template <bool FINAL, bool TC, bool VAR, bool TMA>
-__global__ void __launch_bounds__(128, filter_ctas_per_sm<FINAL, TC, VAR, TMA>())
+template <bool FINAL, bool TC, bool VAR, int SC>
+__global__ void __launch_bounds__(128, filter_ctas_per_sm<FINAL, TC, VAR, SC>())
     filter_kernel(FilterParams prm, const __grid_constant__ CUtensorMap map) {
     extern __shared__ __align__(128) float fsm[];
-    filter_cta<FINAL, TC, VAR, TMA>(prm, &map, blockIdx.x, fsm);
+    filter_cta<FINAL, TC, VAR, SC>(prm, &map, blockIdx.x, fsm);
 }
 
 // Persistent form over a batch of clips: resident CTAs take CTA-sized group
 // ranges from a shared counter, clip-major. TMA: every clip has a tensor map.
 template <bool FINAL, bool TMA>
-__global__ void __launch_bounds__(128, filter_ctas_per_sm<FINAL, false, false, true>())
+__global__ void __launch_bounds__(128, filter_ctas_per_sm<FINAL, false, false, kScatterBoxes>())
     filter_batch_kernel(FilterBatch b) {
     extern __shared__ __align__(128) float fsm[];
     __shared__ FilterParams ps;
@@ -703,7 +729,7 @@ __global__ void __launch_bounds__(128, filter_ctas_per_sm<FINAL, false, false, t
         }
         if (threadIdx.x == 0) ps = b.clips[lo];
         __syncthreads();
-        filter_cta<FINAL, false, false, TMA>(ps, TMA ? b.maps + lo : nullptr,
+        filter_cta<FINAL, false, false, TMA ? kScatterBoxes : kScatterLsu>(ps, TMA ? b.maps + lo : nullptr,
                                              item - b.item_off[lo], fsm);
         __syncthreads();
     }
@@ -883,13 +909,13 @@ __global__ void vaggregate_kernel(VAggregateParams p) {
 
 namespace {
 
-template <bool FINAL, bool TC, bool VAR, bool TMA>
+template <bool FINAL, bool TC, bool VAR, int SC>
 cudaError_t launch_filter_t(const FilterParams &p, const CUtensorMap &map, dim3 grid,
                             cudaStream_t stream) {
     // opt in to more than 48 KB of dynamic shared memory once per device
     static int configured[64] = {};
-    const auto fn = filter_kernel<FINAL, TC, VAR, TMA>;
-    constexpr size_t smem = filter_smem<FINAL, TC, TMA>();
+    const auto fn = filter_kernel<FINAL, TC, VAR, SC>;
+    constexpr size_t smem = filter_smem<FINAL, TC, SC>();
     cudaError_t e = raise_smem_limit(configured, (const void *)fn, smem);
     if (e != cudaSuccess) return e;
     fn<<<grid, 128, smem, stream>>>(p, map);
@@ -900,11 +926,14 @@ template <bool TC, bool VAR>
 cudaError_t launch_filter_form(const FilterParams &p, bool final_, dim3 grid,
                                cudaStream_t stream) {
     CUtensorMap map{};
-    if (scatter_map(p, &map))
-        return final_ ? launch_filter_t<true, TC, VAR, true>(p, map, grid, stream)
-                      : launch_filter_t<false, TC, VAR, true>(p, map, grid, stream);
-    return final_ ? launch_filter_t<true, TC, VAR, false>(p, map, grid, stream)
-                  : launch_filter_t<false, TC, VAR, false>(p, map, grid, stream);
+    if (!scatter_map(p, &map))
+        return final_ ? launch_filter_t<true, TC, VAR, kScatterLsu>(p, map, grid, stream)
+                      : launch_filter_t<false, TC, VAR, kScatterLsu>(p, map, grid, stream);
+    if (p.corner_weight)
+        return final_ ? launch_filter_t<true, TC, VAR, kScatterBoxes>(p, map, grid, stream)
+                      : launch_filter_t<false, TC, VAR, kScatterBoxes>(p, map, grid, stream);
+    return final_ ? launch_filter_t<true, TC, VAR, kScatterWeights>(p, map, grid, stream)
+                  : launch_filter_t<false, TC, VAR, kScatterWeights>(p, map, grid, stream);
 }
 
 }  // namespace
@@ -925,7 +954,7 @@ bool scatter_map(const FilterParams &p, CUtensorMap *map) {
     }();
     // the box starts on a 16-byte boundary of its row; pair indices are exact
     // below 2^20, and rows are 32-bit coordinates
-    if (!encode || !p.corner_weight || !p.acc_base || p.acc_stride % 4 != 0 ||
+    if (!encode || !p.acc_base || (!p.corner_weight && p.mult) || p.acc_stride % 4 != 0 ||
         reinterpret_cast<unsigned long long>(p.acc_base) % 16 != 0 || p.acc_pairs >= (1 << 20) ||
         (long long)p.acc_pairs * p.acc_pair_rows > 0x7fffffffLL)
         return false;
@@ -978,7 +1007,7 @@ template <bool FINAL, bool TMA>
 cudaError_t launch_filter_batch_t(const FilterBatch &b, cudaStream_t stream, int ctas_per_sm) {
     static int configured[64] = {};
     const auto fn = filter_batch_kernel<FINAL, TMA>;
-    constexpr size_t smem = filter_smem<FINAL, false, TMA>();
+    constexpr size_t smem = filter_smem<FINAL, false, TMA ? kScatterBoxes : kScatterLsu>();
     cudaError_t e = raise_smem_limit(configured, (const void *)fn, smem);
     if (e != cudaSuccess) return e;
     fn<<<persistent_grid((const void *)fn, 128, smem, ctas_per_sm), 128, smem, stream>>>(b);

@@ -189,6 +189,16 @@ inline void set_acc_pairs(FilterParams &p, float *base, int pairs, int rows) {
     p.acc_pair_inv = 1.0f / ((float)p.acc_pair_rows * (float)p.acc_stride);
 }
 
+// The same for raw stacks: `stacks` of stack_floats floats each, the plane's
+// pairs from `first` on. Nothing is set where the pairs of other planes do not
+// line up with this plane's (odd subsampled heights).
+inline void set_raw_pairs(FilterParams &p, float *base, long long stacks, long long stack_floats,
+                          long long first, int rows) {
+    const long long pair = 2LL * rows * p.acc_stride, pairs = stacks * (stack_floats / pair);
+    if (stack_floats % pair == 0 && first % pair == 0 && pairs < (1 << 20))
+        set_acc_pairs(p, base, (int)pairs, rows);
+}
+
 cudaError_t launch_filter(const FilterParams &p, bool final_, cudaStream_t stream);
 // The tensor map of the accumulators for the scatter by TMA; false where the
 // launch cannot use it.
