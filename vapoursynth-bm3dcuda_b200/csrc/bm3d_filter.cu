@@ -884,25 +884,64 @@ __global__ void __launch_bounds__(kAggThreads) aggregate_batch_kernel(AggregateB
     }
 }
 
-__global__ void vaggregate_kernel(VAggregateParams p) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+// One V-pixel quad (or single pixel) per thread; the stacks of up to 5 slots are
+// loaded before the first sum needs them.
+template <int V>
+__global__ void __launch_bounds__(128) vaggregate_kernel(VAggregateParams p) {
+    const int x = (blockIdx.x * blockDim.x + threadIdx.x) * V;
     const int y = blockIdx.y;
     const int k = blockIdx.z;
     if (x >= p.width) return;
     const int n = p.n0 + k;
     const int tw = 2 * p.radius + 1;
-    float sw = 0.0f, sv = 0.0f;
-    for (int i = 0; i < tw; ++i) {
+    const size_t slab = (size_t)p.height * p.raw_stride;
+    auto stack = [&](int i) {
         // replication padding at the clip ends (source/source.cpp:832-836)
         const int s = min(max(2 * p.radius - i, n - p.num_frames + 1 + p.radius), n + p.radius);
         const float *f = p.base ? p.base + (size_t)min(max(n - p.radius + i, 0), p.num_frames - 1) *
                                               p.raw_frame_floats
                                 : p.vf[i];
-        const float *a = f + ((size_t)s * 2 * p.height + y) * p.raw_stride + x;
-        sv = __fadd_rn(sv, a[0]);
-        sw = __fadd_rn(sw, a[(size_t)p.height * p.raw_stride]);
+        return f + 2 * (size_t)s * slab + (size_t)y * p.raw_stride + x;
+    };
+    float sv[V] = {}, sw[V] = {};
+    for (int i0 = 0; i0 < tw; i0 += 5) {
+        float a[5][V], w[5][V];
+#pragma unroll
+        for (int j = 0; j < 5; ++j) {
+            if (i0 + j >= tw) break;
+            const float *src = stack(i0 + j);
+            if constexpr (V == 4) {
+                const float4 u = __ldg(reinterpret_cast<const float4 *>(src));
+                const float4 t = __ldg(reinterpret_cast<const float4 *>(src + slab));
+                a[j][0] = u.x; a[j][1] = u.y; a[j][2] = u.z; a[j][3] = u.w;
+                w[j][0] = t.x; w[j][1] = t.y; w[j][2] = t.z; w[j][3] = t.w;
+            } else {
+                a[j][0] = __ldg(src);
+                w[j][0] = __ldg(src + slab);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 5; ++j) {
+            if (i0 + j >= tw) break;
+#pragma unroll
+            for (int c = 0; c < V; ++c) {
+                sv[c] = __fadd_rn(sv[c], a[j][c]);
+                sw[c] = __fadd_rn(sw[c], w[j][c]);
+            }
+        }
     }
-    p.dst[k * p.dst_plane_stride + (size_t)y * p.dst_stride + x] = __fdiv_rn(sv, sw);
+    float *dst = p.dst + k * p.dst_plane_stride + (size_t)y * p.dst_stride + x;
+    float q[V];
+#pragma unroll
+    for (int c = 0; c < V; ++c) q[c] = __fdiv_rn(sv[c], sw[c]);
+    if (V == 4 && x + 4 <= p.width) {
+        *reinterpret_cast<float4 *>(dst) = make_float4(q[0], q[V > 1 ? 1 : 0], q[V > 2 ? 2 : 0],
+                                                       q[V > 3 ? 3 : 0]);
+    } else {
+#pragma unroll
+        for (int c = 0; c < V; ++c)
+            if (x + c < p.width) dst[c] = q[c];
+    }
 }
 
 }  // namespace
@@ -1066,8 +1105,21 @@ cudaError_t launch_aggregate(const AggregateParams &p, cudaStream_t stream) {
 
 cudaError_t launch_vaggregate(const VAggregateParams &p, cudaStream_t stream) {
     if (p.nout == 0) return cudaSuccess;
-    dim3 block(128), grid((p.width + 127) / 128, p.height, p.nout);
-    vaggregate_kernel<<<grid, block, 0, stream>>>(p);
+    // quads where every row of every stack starts on 16 bytes (rows then have
+    // room for the last quad, the stride being a multiple of 4)
+    unsigned long long align = reinterpret_cast<unsigned long long>(p.dst) |
+                               reinterpret_cast<unsigned long long>(p.base);
+    if (!p.base)
+        for (int i = 0; i < 2 * p.radius + 1; ++i)
+            align |= reinterpret_cast<unsigned long long>(p.vf[i]);
+    const bool quads = align % 16 == 0 && p.raw_stride % 4 == 0 && p.dst_stride % 4 == 0 &&
+                       p.raw_frame_floats % 4 == 0 && p.dst_plane_stride % 4 == 0;
+    const int per_block = quads ? 512 : 128;
+    const dim3 block(128), grid((p.width + per_block - 1) / per_block, p.height, p.nout);
+    if (quads)
+        vaggregate_kernel<4><<<grid, block, 0, stream>>>(p);
+    else
+        vaggregate_kernel<1><<<grid, block, 0, stream>>>(p);
     return cudaGetLastError();
 }
 
