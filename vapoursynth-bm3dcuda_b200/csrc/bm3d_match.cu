@@ -71,8 +71,8 @@ int pick_pitch(int base, int block_step, int log_lanes) {
 
 // A warp's match lists: 16 words per thread (SMALL), else 8.
 constexpr size_t kSmallListBytes = 16 * 32 * sizeof(int), kListBytes = 8 * 32 * sizeof(int);
-// Three CTAs per SM: 228 KB less 1 KB per CTA that the hardware reserves.
-constexpr size_t kThirdOfSmem = 75 * 1024;
+// Shared memory of an SM; the hardware reserves 1 KB of it per CTA.
+constexpr size_t kSmemPerSm = 228 * 1024;
 
 }  // namespace
 
@@ -109,7 +109,10 @@ void choose_pitches(MatchGeometry &g, int block_step, int bm_range, int radius, 
     // 2 meet 4-way bank conflicts at an arbitrary pitch)
     const int pitch = pick_pitch(g.pitch, block_step, 0);
     const size_t smem = (size_t)pitch * g.tile_rows * sizeof(float) + lists * g.wx;
-    if (smem <= kThirdOfSmem) {
+    const auto resident = [&](size_t bytes) {
+        return std::min<size_t>(12 / g.wx, kSmemPerSm / (bytes + 1024));
+    };
+    if (smem <= kMatchSmemMax && resident(smem) == resident(g.smem)) {
         g.pitch = pitch;
         g.smem = smem;
     }
@@ -135,26 +138,34 @@ MatchGeometry match_geometry(int width, int height, int block_step, int bm_range
                              int ps_num, int ps_range) {
     const int ws = 2 * bm_range + 1, wt = 2 * ps_range + 1;
     MatchGeometry g{};
-    // the widest CTA (in warps) whose tile fits comfortably
-    if (radius == 0 || ps_num <= 2) {
-        const int spatial[] = {8, 9, 10, 11};
-        const int ks = choose_strip_width(ws, spatial);
-        const int kt = radius == 0 ? 9 : temporal_strip_width(ps_range);
+    const bool small = radius == 0 || ps_num <= 2;
+    // the CTA width with the most resident warps, the widest of equals (8 windows
+    // of 1920x1080, radius 2, bm_range 16: two CTAs of 4 warps on an SM 2.88 ms,
+    // three of 2 warps 3.7)
+    auto widest = [&](int ks, int kt, bool two_entries) {
+        MatchGeometry best{};
+        int best_warps = 0;
         for (int wx = 4; wx >= 1; wx /= 2) {
-            g = match_geometry_with(width, height, block_step, bm_range, radius, ps_range, wx, ks,
-                                    kt, true);
-            if (g.smem <= kThirdOfSmem) break;
+            const MatchGeometry t = match_geometry_with(width, height, block_step, bm_range,
+                                                        radius, ps_range, wx, ks, kt, two_entries);
+            const int warps =
+                std::min<int>(12, (int)(kSmemPerSm / (t.smem + 1024)) * wx);
+            if (warps > best_warps || best.wx == 0) {
+                best_warps = warps;
+                best = t;
+            }
         }
-        if (g.smem <= 200 * 1024) {
-            choose_pitches(g, block_step, bm_range, radius, ps_range);
-            return g;
-        }
+        return best;
+    };
+    if (small) {
+        const int spatial[] = {8, 9, 10, 11};
+        g = widest(choose_strip_width(ws, spatial), radius == 0 ? 9 : temporal_strip_width(ps_range),
+                   true);
     }
-    const int K = choose_strip_width(ws, wt, radius, 2);
-    for (int wx = 4; wx >= 1; wx /= 2) {
-        g = match_geometry_with(width, height, block_step, bm_range, radius, ps_range, wx, K, K,
-                                false);
-        if (match_range_bytes(block_step, bm_range, radius, ps_range, wx, K) <= 72 * 1024) break;
+    // a range that only just fits keeps to the strips that need the least room
+    if (!small || g.smem > 200 * 1024) {
+        const int K = choose_strip_width(ws, wt, radius, 2);
+        g = widest(K, K, false);
     }
     choose_pitches(g, block_step, bm_range, radius, ps_range);
     return g;
@@ -172,9 +183,10 @@ long long match_tiles(const MatchGeometry &g, int nwin) {
 namespace {
 
 // Lanes per reference block: one, unless the launch leaves most of the GPU's
-// 148 x 12 resident warps idle. More lanes shorten each thread's scan and cost
-// insertions (every lane fills a list of its own) and a merge. Times with 1, 4
-// and 8 lanes, us:
+// 148 x 12 resident warps idle, or the search range lets an SM hold only one
+// CTA of four warps with one lane per block (the split tiles hold 32 blocks, not
+// 128). More lanes shorten each thread's scan and cost insertions (every lane
+// fills a list of its own) and a merge. Times with 1, 4 and 8 lanes, us:
 //   120 warps (640x360, radius 0)      74   27   24
 //   224 warps (640x360 step 6, r 2)   250  111   95
 //   288 warps (960x540, r 1)          136   66   83
@@ -182,12 +194,17 @@ namespace {
 //   480 warps (1280x720, r 0)          74   61   65
 //   480 warps (1280x720, r 3)         195  152  173
 //   880 warps (1760x990, r 1)         191  171  221
-//   960 warps (8 x 640x360, r 0)      103  103  113
 //   1020 warps (1920x1080, r 2)       275  304  391
+//   1840 warps (2560x1440, r 0)       187  175
+//   2040 warps (2 x 1920x1080, r 0)   189  189  235
+//   one CTA per SM: 2 x 1920x1080, r 3, bm_range 16, ps_range 6   2417  1707
+//                   2 x 1280x720, r 2, bm_range 20, ps_range 8    1329   926
 int match_lanes(const MatchParams &p, const MatchGeometry &g, int nwin) {
     const long long warps =
         (long long)((p.nbx + 3) / 4) * ((p.nby + 7) / 8) * nwin;  // of 4 x 8 blocks
-    return warps <= 256 ? 8 : warps <= 900 ? 4 : 1;
+    if (warps <= 256) return 8;
+    if (warps <= (p.radius == 0 ? 1850 : 900)) return 4;
+    return kSmemPerSm / (g.smem + 1024) * g.wx <= 4 && g.split[0].smem < g.smem / 2 ? 4 : 1;
 }
 
 }  // namespace
