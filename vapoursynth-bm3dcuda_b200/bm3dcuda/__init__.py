@@ -223,6 +223,11 @@ class _Engine:
             pass
 
     def pack(self, clip: Clip) -> np.ndarray:
+        # a single plane whose rows already have the engine's pitch is read in place
+        pl = clip.planes[0]
+        if (len(clip.planes) == 1 and pl.dtype == np.float32 and pl.shape[2] == self.stride
+                and pl.flags.c_contiguous):
+            return pl.reshape(pl.shape[0], -1)
         buf = np.zeros((clip.num_frames, self.frame_floats), np.float32)
         off = 0
         for pl in clip.planes:
@@ -249,7 +254,7 @@ class _Engine:
         hs = self.pack(src)
         hr = self.pack(ref) if ref is not None else None
         n = src.num_frames
-        dst = np.zeros((n, self.raw_frame_floats if raw else self.frame_floats), np.float32)
+        dst = np.empty((n, self.raw_frame_floats if raw else self.frame_floats), np.float32)
         _lib.check(L.bm3d_b200_clip_run_host(
             self.h, hs.ctypes.data, hr.ctypes.data if hr is not None else None, dst.ctypes.data,
             _lib.DST_RAW if raw else _lib.DST_AGGREGATED, None))
@@ -378,7 +383,7 @@ def twostage(clip: Clip, **kw) -> Clip:
     eng = _Engine(clip, a)
     try:
         hs = eng.pack(clip)
-        dst = np.zeros_like(hs)
+        dst = np.empty_like(hs)
         _lib.check(_lib.lib().bm3d_b200_clip_twostage_host(eng.h, hs.ctypes.data, dst.ctypes.data,
                                                            None))
         planes = eng.unpack(dst, raw=False)
