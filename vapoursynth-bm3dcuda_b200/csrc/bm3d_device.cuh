@@ -499,6 +499,35 @@ __device__ __forceinline__ void list_insert_n(List8 &l, float err, int pos) {
     l.e[0] = fminf(l.e[0], err);
 }
 
+// A stage's match list while its candidates are scanned. `thr` is the distance
+// a candidate must be below to enter.
+//
+// The scan is register-bound: 64 registers hold the reference block, and the
+// strip's sums need as many as they can get to run their chains side by side
+// (a CTA alone scans a radius-0 tile in 82 us at 168 registers with the lists
+// in registers, 66 us at 224). So the 8-entry list lies in shared memory, one
+// column per thread (distances, then positions), and is read and written back
+// only by strips that improve it.
+struct ColumnList {
+    float *col;  // this thread's column, entries `pitch` words apart
+    int pitch;
+    float thr;
+
+    __device__ __forceinline__ void load(List8 &l) const {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) l.e[i] = col[i * pitch];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) l.p[i] = __float_as_int(col[(8 + i) * pitch]);
+    }
+    __device__ __forceinline__ void store(const List8 &l) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) col[i * pitch] = l.e[i];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) col[(8 + i) * pitch] = __int_as_float(l.p[i]);
+        thr = l.e[7];
+    }
+};
+
 // Register-array element at a runtime index without local-memory indexing.
 template <int N, typename T>
 __device__ __forceinline__ T pick(const T (&a)[N], int i) {

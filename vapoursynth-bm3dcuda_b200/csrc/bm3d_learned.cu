@@ -109,16 +109,19 @@ __device__ __forceinline__ CellRect cell_rect(const Box &b) {
 // Ranks the cells of search window i of a stage into `keys`, skipping cells
 // that an earlier window's cell rectangle already held (b0: window 0's box;
 // windows 1 .. i-1 are recomputed from their centres in `last`). ord0: the
-// ordinal of the window's first cell. The window's cell rows are walked one
-// by one, four cells per iteration with their loads issued first; a skipped
-// cell inserts the empty key (a no-op of the min/max network), so the walk
-// has no divergent branch.
-template <int K>
+// ordinal of the window's first cell. The cells are walked in order, kRankBatch
+// at a time with their loads issued first (30 windows of 1920x1080, radius 2:
+// 1.96 ms; 1.99 with four loads in flight and single ones for a row's remainder);
+// a skipped cell inserts the empty key (a no-op of the min/max network),
+// so the walk has no divergent branch.
+constexpr int kRankBatch = 8;
+
+template <int K, int N>
 __device__ __forceinline__ void rank_cells(unsigned (&keys)[K], const uint4 er,
                                            const uint4 *__restrict__ emb, int w2, const Box &bi,
                                            unsigned ord0, int i, const Box &b0,
                                            const MatchParams &p, int st, int x, int y, int m,
-                                           int range, const int (&last)[8]) {
+                                           int range, const int (&last)[N]) {
     const CellRect cr = cell_rect(bi);
     const CellRect c0 = cell_rect(b0);
     auto seen_earlier = [&](int gx, int gy) {
@@ -128,29 +131,36 @@ __device__ __forceinline__ void rank_cells(unsigned (&keys)[K], const uint4 er,
             seen |= in_cells(stage_box(p, st, x, y, m, range, pick(last, j)), gx, gy);
         return seen;
     };
-    const int ncol = cr.gx1 - cr.gx0 + 1;
-    unsigned o = ord0;
-    for (int gy = cr.gy0; gy <= cr.gy1; ++gy, o += (unsigned)ncol) {
-        const uint4 *row = cell_ptr(emb, w2, cr.gx0, gy);
-        int k = 0;
-        for (; k + 3 < ncol; k += 4) {
-            uint4 e[4];
+    const int ncol = cr.gx1 - cr.gx0 + 1, n = ncol * (cr.gy1 - cr.gy0 + 1);
+    int gx = cr.gx0, gy = cr.gy0;
+    const uint4 *cell = cell_ptr(emb, w2, gx, gy);
+    for (int c = 0; c < n; c += kRankBatch) {
+        uint4 e[kRankBatch];
+        bool skip[kRankBatch];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) e[j] = __ldg(row + k + j);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const unsigned key = (emb_dist(er, e[j]) << kOrdinalBits) | (o + k + j);
-                key_insert(keys, seen_earlier(cr.gx0 + k + j, gy) ? kNoKey : key);
+        for (int j = 0; j < kRankBatch; ++j) {
+            e[j] = __ldg(cell);
+            skip[j] = c + j >= n || seen_earlier(gx, gy);
+            if (c + j + 1 < n) {  // the last cell is loaded again past the end
+                const bool wrap = gx == cr.gx1;
+                gx = wrap ? cr.gx0 : gx + 1;
+                gy += wrap;
+                cell += wrap ? w2 - ncol + 1 : 1;
             }
         }
-        for (; k < ncol; ++k) {
-            const unsigned key = (emb_dist(er, __ldg(row + k)) << kOrdinalBits) | (o + k);
-            key_insert(keys, seen_earlier(cr.gx0 + k, gy) ? kNoKey : key);
+#pragma unroll
+        for (int j = 0; j < kRankBatch; ++j) {
+            const unsigned key = (emb_dist(er, e[j]) << kOrdinalBits) | (ord0 + c + j);
+            key_insert(keys, skip[j] ? kNoKey : key);
         }
     }
 }
 
-template <int K>
+// SMALL (ps_num <= 2, or no neighbour frames): a neighbour frame's list keeps
+// two entries, all that is ever read of it, and the block's list lies in shared
+// memory while a stage ranks and scores (168 registers: 412 bytes spilled
+// before, 132 now).
+template <int K, bool SMALL>
 __device__ void learned_tile(const MatchParams &p, const LearnedParams &lp, int tile_x,
                              int tile_y, int win, float *tile) {
     const int lane = threadIdx.x & 31;
@@ -182,8 +192,11 @@ __device__ void learned_tile(const MatchParams &p, const LearnedParams &lp, int 
     uint4 er = make_uint4(0, 0, 0, 0);
     List8 list;
     list_init(list, FLT_MAX, pack_pos(x, y, center));
-    int *center_pos = reinterpret_cast<int *>(tile + (size_t)p.pitch * p.tile_rows) + threadIdx.x;
-    int last[8];
+    // the block's list (SMALL), else the spatial list's positions, which seed
+    // the +1 direction
+    ColumnList cl{tile + (size_t)p.pitch * p.tile_rows + threadIdx.x, (int)blockDim.x, 0.0f};
+    constexpr int kLast = SMALL ? 2 : 8;
+    int last[kLast], near[kLast];  // window centres; the spatial stage's, SMALL
 
     for (int st = 0; st <= 2 * r; ++st) {
         const int t = st <= r ? st : st - r;
@@ -209,7 +222,8 @@ __device__ void learned_tile(const MatchParams &p, const LearnedParams &lp, int 
         if (!active) continue;
         if (st == r + 1) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) last[i] = center_pos[i * blockDim.x];
+            for (int i = 0; i < kLast; ++i)
+                last[i] = SMALL ? near[i] : __float_as_int(cl.col[i * cl.pitch]);
         }
         const int range = st == 0 ? p.bm_range : p.ps_range;
         const int nwin = st == 0 ? 1 : p.ps_num;
@@ -263,28 +277,44 @@ __device__ void learned_tile(const MatchParams &p, const LearnedParams &lp, int 
 #pragma unroll
                 for (int du = 0; du < 2; ++du) {
                     const int cu = u + du, cv = v + dv;
-                    if (cu >= bw.l && cu <= bw.r && cv >= bw.t && cv <= bw.b &&
-                        err[du] < fl.e[7])
-                        list_insert(fl, err[du], pack_pos(cu, cv, z));
+                    if (cu >= bw.l && cu <= bw.r && cv >= bw.t && cv <= bw.b) {
+                        const int pos = pack_pos(cu, cv, z);
+                        if (SMALL && st > 0)
+                            list_insert_n<2>(fl, err[du], pos);
+                        else if (err[du] < fl.e[7])
+                            list_insert_n<8>(fl, err[du], pos);
+                    }
                 }
             }
         }
 
         if (st == 0) {
-            list = fl;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) center_pos[i * blockDim.x] = last[i] = fl.p[i];
-        } else {
-            for (int i = 0; i < p.ps_num; ++i) {
-                const float e = pick(fl.e, i);
-                if (e < list.e[7]) list_insert(list, e, pick(fl.p, i));
+            for (int i = 0; i < kLast; ++i) last[i] = fl.p[i];
+            if (SMALL) {
+                cl.store(fl);
+#pragma unroll
+                for (int i = 0; i < kLast; ++i) near[i] = fl.p[i];
+            } else {
+                list = fl;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) cl.col[i * cl.pitch] = __int_as_float(fl.p[i]);
             }
+        } else {
+            if (SMALL) cl.load(list);
+            for (int i = 0; i < p.ps_num; ++i) {
+                const float e = SMALL ? (i == 0 ? fl.e[0] : fl.e[1]) : pick(fl.e, i);
+                const int pos = SMALL ? (i == 0 ? fl.p[0] : fl.p[1]) : pick(fl.p, i);
+                if (e < list.e[7]) list_insert_n<8>(list, e, pos);
+            }
+            if (SMALL) cl.store(list);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) last[i] = fl.p[i];
+            for (int i = 0; i < kLast; ++i) last[i] = fl.p[i];
         }
     }
 
     if (!active) return;
+    if (SMALL) cl.load(list);
 
     const int cpos = pack_pos(x, y, center);
     const int blk = by * p.nbx + bx;
@@ -317,12 +347,12 @@ __device__ void learned_tile(const MatchParams &p, const LearnedParams &lp, int 
 // band of tile rows in every window before the next band, so the CTAs that
 // run together read the same rows of the (shared) frames and embeddings and
 // those stay in L2 (window-major order re-reads them from DRAM).
-template <int K>
+template <int K, bool SMALL>
 __global__ void __launch_bounds__(128, 3) learned_match_kernel(MatchParams p, LearnedParams lp) {
     extern __shared__ float tile[];
     const unsigned id = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
     const unsigned rest = id / gridDim.x;
-    learned_tile<K>(p, lp, (int)(id % gridDim.x), (int)(rest / gridDim.z),
+    learned_tile<K, SMALL>(p, lp, (int)(id % gridDim.x), (int)(rest / gridDim.z),
                     p.win0 + (int)(rest % gridDim.z), tile);
 }
 
@@ -584,21 +614,37 @@ cudaError_t launch_rescore(const MatchParams &p, int nwin, cudaStream_t stream) 
 }
 
 MatchGeometry learned_geometry(int width, int height, int block_step, int bm_range, int radius,
-                               int ps_range) {
+                               int ps_num, int ps_range) {
     MatchGeometry g{};
     g.nbx = (width - 8 + block_step - 1) / block_step + 1;
     g.nby = (height - 8 + block_step - 1) / block_step + 1;
     const int mmax = bm_range + radius * ps_range;
-    for (int wx = 4; wx >= 1; wx /= 2) {
-        const int tw = (4 * wx - 1) * block_step + 2 * mmax + 10;
-        const int th = 7 * block_step + 2 * mmax + 10;
-        g.wx = wx;
-        g.pitch = tw + 8;
-        g.tile_rows = th;
-        g.smem = (size_t)g.pitch * th * sizeof(float) + 8 * 32 * wx * sizeof(int);
-        if (g.smem <= 72 * 1024) break;
-    }
+    g.tile_rows = 7 * block_step + 2 * mmax + 10;
     g.ks = g.kt = 2;
+    g.small = radius == 0 || ps_num <= 2;
+    auto bytes = [&](int pitch, int wx, int words) {
+        return (size_t)pitch * g.tile_rows * sizeof(float) + (size_t)words * 32 * wx * sizeof(int);
+    };
+    // a range whose one-warp CTA needs more than 220 KB (with 8 list words per
+    // thread) is refused
+    if (bytes(3 * block_step + 2 * mmax + 18, 1, 8) > kMatchSmemLimit) {
+        g.wx = 1;
+        g.smem = kMatchSmemMax + 1;
+        return g;
+    }
+    // the CTA width with the most resident warps, the widest of equals
+    int best = 0;
+    for (int wx = 4; wx >= 1; wx /= 2) {
+        const int pitch = (4 * wx - 1) * block_step + 2 * mmax + 17;
+        const size_t smem = bytes(pitch, wx, g.small ? 16 : 8);
+        const int warps = std::min<int>(12, (int)(228 * 1024 / (smem + 1024)) * wx);
+        if (warps > best && smem <= kMatchSmemMax) {
+            best = warps;
+            g.wx = wx;
+            g.pitch = pitch;
+            g.smem = smem;
+        }
+    }
     return g;
 }
 
@@ -609,26 +655,35 @@ bool learned_ordinals_fit(int bm_range, int ps_num, int ps_range) {
     return sp <= (1 << kOrdinalBits) && tp <= (1 << kOrdinalBits);
 }
 
-template <int K>
+template <int K, bool SMALL>
 cudaError_t launch_learned_k(const MatchParams &p, const LearnedParams &lp, const MatchGeometry &g,
                              int nwin, cudaStream_t stream) {
     static int configured[64] = {0};
-    cudaError_t e = raise_smem_limit(configured, (const void *)learned_match_kernel<K>, g.smem);
+    cudaError_t e =
+        raise_smem_limit(configured, (const void *)learned_match_kernel<K, SMALL>, g.smem);
     if (e != cudaSuccess) return e;
     dim3 block(32 * g.wx);
     dim3 grid((p.nbx + 4 * g.wx - 1) / (4 * g.wx), (p.nby + 7) / 8, nwin);
-    learned_match_kernel<K><<<grid, block, g.smem, stream>>>(p, lp);
+    learned_match_kernel<K, SMALL><<<grid, block, g.smem, stream>>>(p, lp);
     return cudaGetLastError();
+}
+
+template <bool SMALL>
+cudaError_t launch_learned_s(const MatchParams &p, const LearnedParams &lp, const MatchGeometry &g,
+                             int nwin, cudaStream_t stream) {
+    const int cells = std::max(lp.cells_s, lp.cells_t);
+    if (cells <= 2) return launch_learned_k<2, SMALL>(p, lp, g, nwin, stream);
+    return cells <= 4 ? launch_learned_k<4, SMALL>(p, lp, g, nwin, stream)
+                      : launch_learned_k<8, SMALL>(p, lp, g, nwin, stream);
 }
 
 cudaError_t launch_learned_match(const MatchParams &p, const LearnedParams &lp,
                                  const MatchGeometry &g, int nwin, cudaStream_t stream) {
-    if (g.smem > 220 * 1024 || lp.cells_s < 1 || lp.cells_s > 8 || lp.cells_t < 1 ||
+    if (g.smem > kMatchSmemMax || lp.cells_s < 1 || lp.cells_s > 8 || lp.cells_t < 1 ||
         lp.cells_t > 8 || !learned_ordinals_fit(p.bm_range, p.ps_num, p.ps_range))
         return cudaErrorInvalidValue;
-    if (std::max(lp.cells_s, lp.cells_t) <= 2) return launch_learned_k<2>(p, lp, g, nwin, stream);
-    return std::max(lp.cells_s, lp.cells_t) <= 4 ? launch_learned_k<4>(p, lp, g, nwin, stream)
-                                                 : launch_learned_k<8>(p, lp, g, nwin, stream);
+    return g.small ? launch_learned_s<true>(p, lp, g, nwin, stream)
+                   : launch_learned_s<false>(p, lp, g, nwin, stream);
 }
 
 cudaError_t launch_match_fallback(const MatchParams &p, const unsigned *list,
