@@ -17,13 +17,15 @@ def window(h, w, radius, kind, seed):
     return frames[None]
 
 
-# blocks per launch: 8 lanes up to 256 warps of 4 x 8 blocks, 4 up to 900, then 1
+# warps of 4 x 8 blocks per launch choose the form
 SIZES = [
     (8, 8, 8),        # one block
     (41, 67, 8),      # clamped last blocks, a few warps
-    (120, 97, 2),     # 57 x 46 blocks
-    (100, 260, 1),    # 4 lanes: 253 x 93 blocks
-    (163, 203, 1),    # one lane: 196 x 156 blocks = 980 warps
+    (120, 97, 2),     # 96 warps: 8 lanes per block
+    (100, 90, 1),     # 252: 4 lanes
+    (100, 260, 1),    # 768: one lane, 200 registers
+    (163, 203, 1),    # 980
+    (390, 420, 1),    # 4944: one lane, 168 registers
 ]
 
 

@@ -88,6 +88,8 @@ MatchGeometry match_geometry_with(int width, int height, int block_step, int bm_
 void choose_pitches(MatchGeometry &g, int block_step, int bm_range, int radius, int ps_range);
 // Strip width of the temporal windows (small geometries).
 int temporal_strip_width(int ps_range);
+// Resident CTAs per SM (2 or 3) that a launch of the small search aims at.
+int match_ctas(const MatchGeometry &g, int nwin);
 // CTA tiles of one launch over nwin windows.
 long long match_tiles(const MatchGeometry &g, int nwin);
 cudaError_t launch_match(const MatchParams &p, const MatchGeometry &g, int nwin,

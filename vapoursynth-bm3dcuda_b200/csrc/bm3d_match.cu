@@ -176,6 +176,21 @@ bool match_too_large(int block_step, int bm_range, int radius, int ps_range) {
     return match_range_bytes(block_step, bm_range, radius, ps_range, 1, K) > kMatchSmemLimit;
 }
 
+// Resident CTAs per SM for the small SSD search, one lane per block: times at
+// 168 registers and three CTAs, and at about 200 and two, us:
+//   240 CTAs (8 x 640x360, radius 0)              103    95
+//   255 CTAs (1920x1080, radius 2)                276   251
+//   460 CTAs (2560x1440, radius 0)                187   178
+//   1020 CTAs (3840x2160, radius 0, bm_range 16)  801   791
+//   1080 CTAs (3 x 853x479, step 3)              1609  1554
+//   2040 CTAs (8 x 1920x1080, radius 0)           601   611
+//   3060 CTAs (12 x 1920x1080, radius 2)         2405  2421
+//   2040 CTAs whose tile leaves room for two:
+//     8 x 1920x1080, radius 3                    2405  2135
+int match_ctas(const MatchGeometry &g, int nwin) {
+    return match_tiles(g, nwin) > 1100 && kSmemPerSm / (g.smem + 1024) >= 3 ? 3 : 2;
+}
+
 long long match_tiles(const MatchGeometry &g, int nwin) {
     return (long long)((g.nbx + 4 * g.wx - 1) / (4 * g.wx)) * ((g.nby + 7) / 8) * nwin;
 }
@@ -187,23 +202,21 @@ namespace {
 // CTA of four warps with one lane per block (the split tiles hold 32 blocks, not
 // 128). More lanes shorten each thread's scan and cost insertions (every lane
 // fills a list of its own) and a merge. Times with 1, 4 and 8 lanes, us:
-//   120 warps (640x360, radius 0)      74   27   24
-//   224 warps (640x360 step 6, r 2)   250  111   95
-//   288 warps (960x540, r 1)          136   66   83
-//   336 warps (2 x 333x211, r 1)      323  148  207
-//   480 warps (1280x720, r 0)          74   61   65
-//   480 warps (1280x720, r 3)         195  152  173
-//   880 warps (1760x990, r 1)         191  171  221
-//   1020 warps (1920x1080, r 2)       275  304  391
-//   1840 warps (2560x1440, r 0)       187  175
-//   2040 warps (2 x 1920x1080, r 0)   189  189  235
-//   one CTA per SM: 2 x 1920x1080, r 3, bm_range 16, ps_range 6   2417  1707
-//                   2 x 1280x720, r 2, bm_range 20, ps_range 8    1329   926
+//   120 warps (640x360, radius 0)      65   25   23
+//   224 warps (640x360 step 6, r 2)   183   99  103
+//   288 warps (960x540, r 1)          111   62   80
+//   336 warps (2 x 333x211, r 1)      242  129  171
+//   480 warps (1280x720, r 0)          64   60   69
+//   480 warps (1280x720, r 3)         136  145  181
+//   880 warps (1760x990, r 1)         173  175  230
+//   960 warps (8 x 640x360, r 0)       95  107  123
+//   one CTA per SM: 2 x 1920x1080, r 3, bm_range 16, ps_range 6   1839  1724
+//                   2 x 1280x720, r 2, bm_range 20, ps_range 8    1046   923
 int match_lanes(const MatchParams &p, const MatchGeometry &g, int nwin) {
     const long long warps =
         (long long)((p.nbx + 3) / 4) * ((p.nby + 7) / 8) * nwin;  // of 4 x 8 blocks
-    if (warps <= 256) return 8;
-    if (warps <= (p.radius == 0 ? 1850 : 900)) return 4;
+    if (warps <= 160) return 8;
+    if (warps <= (p.radius == 0 ? 600 : 450)) return 4;
     return kSmemPerSm / (g.smem + 1024) * g.wx <= 4 && g.split[0].smem < g.smem / 2 ? 4 : 1;
 }
 

@@ -10,8 +10,8 @@ namespace {
 // parameters: resident CTAs take CTA tiles from a shared counter, clip-major
 // in the order the clips were added; per-clip parameters are staged in
 // shared memory for the tile.
-template <int K, int KT, bool SMALL>
-__global__ void __launch_bounds__(128, 3) match_batch_kernel(MatchBatch b) {
+template <int K, int KT, bool SMALL, int CTAS>
+__global__ void __launch_bounds__(128, CTAS) match_batch_kernel(MatchBatch b) {
     extern __shared__ float tile[];
     __shared__ MatchParams ps;
     __shared__ long long item_s;
@@ -40,9 +40,9 @@ __global__ void __launch_bounds__(128, 3) match_batch_kernel(MatchBatch b) {
     }
 }
 
-template <int K, int KT, bool SMALL>
+template <int K, int KT, bool SMALL, int CTAS>
 cudaError_t launch_match_batch_t(const MatchBatch &b, int wx, size_t smem, cudaStream_t stream) {
-    auto fn = match_batch_kernel<K, KT, SMALL>;
+    auto fn = match_batch_kernel<K, KT, SMALL, CTAS>;
     static int configured[64] = {0};
     int dev = 0, sms = 0, per_sm = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -60,9 +60,14 @@ cudaError_t launch_match_batch_t(const MatchBatch &b, int wx, size_t smem, cudaS
 template <int K>
 cudaError_t launch_match_batch_k(const MatchBatch &b, int kt, bool small, int wx, size_t smem,
                                  cudaStream_t stream) {
-    if (!small) return launch_match_batch_t<K, K, false>(b, wx, smem, stream);
-    return kt == 11 ? launch_match_batch_t<K, 11, true>(b, wx, smem, stream)
-                    : launch_match_batch_t<K, 9, true>(b, wx, smem, stream);
+    if (!small) return launch_match_batch_t<K, K, false, 2>(b, wx, smem, stream);
+    // the registers for three CTAs per SM where the largest tile leaves room
+    // for them (match_ctas)
+    if (3 * (smem + 1024) <= 228 * 1024)
+        return kt == 11 ? launch_match_batch_t<K, 11, true, 3>(b, wx, smem, stream)
+                        : launch_match_batch_t<K, 9, true, 3>(b, wx, smem, stream);
+    return kt == 11 ? launch_match_batch_t<K, 11, true, 2>(b, wx, smem, stream)
+                    : launch_match_batch_t<K, 9, true, 2>(b, wx, smem, stream);
 }
 
 }  // namespace

@@ -24,15 +24,16 @@
 //     32 threads of a warp hit 32 distinct banks when block_step is 8; for
 //     other steps the row pitch is picked for the fewest conflicts.
 //
-// Bound: the FP32 pipe (143 of its slots per distance; 1.50 ms of distances for
-// 12 windows of 1920x1080, radius 2), then the insertions and the registers:
-// a strip's chains run side by side only as far as registers allow. 12 such
-// windows take 2.43 ms (62% of the pipe), 2.85 before: two-entry temporal
-// lists, strip widths of their own for the temporal windows (9 of 9 columns
-// used instead of 9 of 10) and the spatial list parked in shared memory.
-// Measured and not kept: 4 CTAs per SM at 128 registers (1.10x the time), 2 at
-// 200 (1.02x), both halves of a block's columns as separate strips to skip the
-// second (1.13x).
+// Bound: the FP32 pipe and the issue slots (143 pipe slots per distance; 1.50 ms
+// of distances for 12 windows of 1920x1080, radius 2), then the insertions and
+// the registers: a strip's chains run side by side only as far as registers
+// allow. 12 such windows take 2.41 ms (62% of the pipe), 2.85 before: two-entry
+// temporal lists, strip widths of their own for the temporal windows (9 of 9
+// columns used instead of 9 of 10) and the spatial list parked in shared memory.
+// Measured and not kept: 4 CTAs per SM at 128 registers (1.10x the time), both
+// halves of a block's columns as separate strips to skip the second (1.13x),
+// two lanes per block with half its columns each and twice the warps (1.13x),
+// the 19 columns of a window as one strip (0.98x at radius 0, 1.06x at 2).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -382,16 +383,20 @@ __device__ __forceinline__ void match_tile(const MatchParams &p, int tile_x, int
     out[1] = make_int4(list.p[4], list.p[5], list.p[6], list.p[7]);
 }
 
-template <int K, int KT, int M, int S, bool SMALL>
-__global__ void __launch_bounds__(128, 3) match_kernel(MatchParams p) {
+// CTAS: resident CTAs per SM that the registers aim at. Two (up to 255 registers a
+// thread) run a warp about 20% faster than three (168), which pays until a
+// launch has CTAs enough to fill three places for several waves; match_ctas has
+// the rule.
+template <int K, int KT, int M, int S, bool SMALL, int CTAS>
+__global__ void __launch_bounds__(128, CTAS) match_kernel(MatchParams p) {
     extern __shared__ float tile[];
     match_tile<K, KT, M, S, SMALL>(p, blockIdx.x, blockIdx.y, p.win0 + blockIdx.z, tile);
 }
 
-template <int K, int KT, int M, int S, bool SMALL>
+template <int K, int KT, int M, int S, bool SMALL, int CTAS = 2>
 cudaError_t launch_match_t(const MatchParams &p, dim3 grid, dim3 block, size_t smem,
                            cudaStream_t stream) {
-    auto fn = match_kernel<K, KT, M, S, SMALL>;
+    auto fn = match_kernel<K, KT, M, S, SMALL, CTAS>;
     // The dynamic shared-memory opt-in is per device; raise it only when a
     // launch needs more than this device was configured for, so that launches
     // recorded into CUDA graphs do not repeat the attribute call.
@@ -408,6 +413,9 @@ cudaError_t launch_match_lanes(const MatchParams &p, const MatchGeometry &g, int
     if (lanes == 1) {
         if (g.smem > kMatchSmemMax) return cudaErrorInvalidValue;
         const dim3 grid((p.nbx + 4 * g.wx - 1) / (4 * g.wx), (p.nby + 7) / 8, nwin);
+        if constexpr (SMALL)
+            if (match_ctas(g, nwin) == 3)
+                return launch_match_t<K, KT, 0, 1, true, 3>(p, grid, 32 * g.wx, g.smem, stream);
         return launch_match_t<K, KT, 0, 1, SMALL>(p, grid, 32 * g.wx, g.smem, stream);
     }
     const auto &sp = g.split[lanes == 4 ? 0 : 1];

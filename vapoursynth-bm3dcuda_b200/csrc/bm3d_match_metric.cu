@@ -27,8 +27,13 @@ cudaError_t launch_metric(MatchParams q, const MatchGeometry &g, int nwin, int l
                       : launch_metric<1, M, false>(q, g, nwin, 1, stream);
     const dim3 grid((q.nbx + 4 * wx - 1) / (4 * wx), (q.nby + rows - 1) / rows, nwin);
     const dim3 block(32 * wx * wy);
-    if constexpr (SMALL)
+    if constexpr (SMALL) {
         if (lanes > 1) return launch_match_t<K, K, M, 4, true>(q, grid, block, smem, stream);
+        // three CTAs per SM once there are several waves of them (1020 CTAs, 4 x
+        // 1920x1080: SSD/NORM 648 us, 714 with two; 240 CTAs: 223, 213)
+        if ((long long)grid.x * grid.y * grid.z > 600)
+            return launch_match_t<K, K, M, 1, true, 3>(q, grid, block, smem, stream);
+    }
     return launch_match_t<K, K, M, 1, SMALL>(q, grid, block, smem, stream);
 }
 
