@@ -228,16 +228,26 @@ __device__ __forceinline__ uint32_t pack_bf16(__nv_bfloat16 lo, __nv_bfloat16 hi
     return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
 }
 
+// 2 cos(pi m / 16), m = 0 .. 8
+__constant__ double kTwoCos[9] = {
+    2.0, 1.9615705608064609, 1.8477590650225735,
+    1.6629392246050905, 1.4142135623730951, 1.1111404660392046,
+    0.7653668647301797, 0.39018064403225666, 0.0};
+
 // B fragments of the forward (C) or inverse (C^T) map for this lane: the mma
-// computes out[line][n] = sum_k in[line][k] * B[k][n], B[k][n] = D[n][k].
+// computes out[line][n] = sum_k in[line][k] * B[k][n], B[k][n] = D[n][k]. (From a
+// table: four double-precision cosines per thread cost a tenth of the kernel.)
 __device__ __forceinline__ SplitB dct_fragment(bool forward, int lane) {
     const int n = lane >> 2, t = lane & 3;
     __nv_bfloat16 h[2], m[2], l[2];
+#pragma unroll
     for (int j = 0; j < 2; ++j) {
         const int k = 2 * t + j;
         const int fr = forward ? n : k, ps = forward ? k : n;  // frequency, position
-        const double c = fr == 0 ? 0.70710678118654752440 : 1.0;
-        const double d = 2.0 * c * cos(3.14159265358979323846 * (2 * ps + 1) * fr / 16.0);
+        // the angle pi a / 16, folded into [0, pi / 2]
+        const int a = ((2 * ps + 1) * fr) & 31, b = a > 16 ? 32 - a : a;
+        double d = b > 8 ? -kTwoCos[16 - b] : kTwoCos[b];
+        if (fr == 0) d = 1.41421356237309504880;
         h[j] = __double2bfloat16(d);
         const double r1 = d - (double)__bfloat162float(h[j]);
         m[j] = __double2bfloat16(r1);
@@ -246,12 +256,22 @@ __device__ __forceinline__ SplitB dct_fragment(bool forward, int lane) {
     return SplitB{pack_bf16(h[0], h[1]), pack_bf16(m[0], m[1]), pack_bf16(l[0], l[1])};
 }
 
-__device__ __forceinline__ void split3(float x, __nv_bfloat16 &h, __nv_bfloat16 &m,
-                                       __nv_bfloat16 &l) {
-    h = __float2bfloat16_rn(x);
-    const float r1 = __fsub_rn(x, __bfloat162float(h));
-    m = __float2bfloat16_rn(r1);
-    l = __float2bfloat16_rn(__fsub_rn(r1, __bfloat162float(m)));
+// Two values into three pairs of BF16 parts (x0 in the low halves): each part is
+// the rounding of what the previous ones leave. Conversions two at a time; a
+// part's value is its half word as the top of a float.
+__device__ __forceinline__ uint32_t cvt_bf16x2(float lo, float hi) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+__device__ __forceinline__ float bf16_lo(uint32_t p) { return __uint_as_float(p << 16); }
+__device__ __forceinline__ float bf16_hi(uint32_t p) { return __uint_as_float(p & 0xffff0000u); }
+
+__device__ __forceinline__ void split3(float x0, float x1, uint32_t &h, uint32_t &m, uint32_t &l) {
+    h = cvt_bf16x2(x0, x1);
+    const float r0 = __fsub_rn(x0, bf16_lo(h)), r1 = __fsub_rn(x1, bf16_hi(h));
+    m = cvt_bf16x2(r0, r1);
+    l = cvt_bf16x2(__fsub_rn(r0, bf16_lo(m)), __fsub_rn(r1, bf16_hi(m)));
 }
 
 __device__ __forceinline__ void mma_k8(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b) {
@@ -281,14 +301,9 @@ __device__ __forceinline__ void tc_pass(float *W, int axis, const SplitB &B, int
             const int l0 = mt * 16 + gq, l1 = l0 + 8;
             const int o00 = tc_addr(axis, l0, 2 * t), o01 = tc_addr(axis, l0, 2 * t + 1);
             const int o10 = tc_addr(axis, l1, 2 * t), o11 = tc_addr(axis, l1, 2 * t + 1);
-            __nv_bfloat16 h[4], m[4], l[4];
-            split3(G[o00], h[0], m[0], l[0]);
-            split3(G[o01], h[1], m[1], l[1]);
-            split3(G[o10], h[2], m[2], l[2]);
-            split3(G[o11], h[3], m[3], l[3]);
-            const uint32_t ah0 = pack_bf16(h[0], h[1]), ah1 = pack_bf16(h[2], h[3]);
-            const uint32_t am0 = pack_bf16(m[0], m[1]), am1 = pack_bf16(m[2], m[3]);
-            const uint32_t al0 = pack_bf16(l[0], l[1]), al1 = pack_bf16(l[2], l[3]);
+            uint32_t ah0, am0, al0, ah1, am1, al1;
+            split3(G[o00], G[o01], ah0, am0, al0);
+            split3(G[o10], G[o11], ah1, am1, al1);
             float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
             mma_k8(acc, al0, al1, B.h);
             mma_k8(acc, am0, am1, B.m);
