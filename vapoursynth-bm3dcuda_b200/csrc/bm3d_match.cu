@@ -50,7 +50,8 @@ int pick_pitch(int base, int block_step, int log_lanes) {
     int best = base, best_cost = 1 << 30;
     for (int pitch = base; pitch < base + 16 && best_cost > 8; ++pitch) {
         int cost = 0;
-        for (int phase = 0; phase < 8; ++phase) {
+        // a phase costs at least 1: stop where the pitch cannot win any more
+        for (int phase = 0; phase < 8 && cost + 8 - phase < best_cost; ++phase) {
             unsigned char hits[32] = {};
             int worst = 0;
             for (int l = 0; l < 32; ++l) {
@@ -60,6 +61,7 @@ int pick_pitch(int base, int block_step, int log_lanes) {
                 worst = std::max(worst, (int)++hits[bank]);
             }
             cost += worst;
+            if (phase < 7 && cost + 7 - phase >= best_cost) cost = best_cost;
         }
         if (cost < best_cost) {
             best_cost = cost;
