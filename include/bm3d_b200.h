@@ -554,6 +554,14 @@ BM3D_B200_API int bm3d_b200_clip_learned_stats(bm3d_b200_clip *c, long long *blo
 BM3D_B200_API int bm3d_b200_selftest_reciprocal(unsigned lo_bits, unsigned hi_bits,
                                                 unsigned long long *mismatches,
                                                 unsigned *first_bad);
+/* The form a block-matching launch over `windows` windows takes: *lanes lanes
+ * per reference block and CTAs of *shared_bytes of shared memory, of which
+ * *limit_bytes fit. BM3D_B200_ERR_UNSUPPORTED (or _INVALID) for searches that
+ * are refused. Host arithmetic only: no device is touched. */
+BM3D_B200_API int bm3d_b200_selftest_match_plan(int width, int height, int block_step,
+                                                int bm_range, int radius, int ps_num,
+                                                int ps_range, int windows, int *lanes,
+                                                long long *shared_bytes, long long *limit_bytes);
 
 #ifdef __cplusplus
 }

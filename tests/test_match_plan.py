@@ -1,0 +1,52 @@
+"""Every search that is accepted has a launch that fits on chip: the range check
+keeps to one-warp CTAs of at most 220 KB, and the form picked for a launch stays
+within a CTA's 227 KB. No device is needed."""
+import ctypes
+
+import pytest
+
+OK, UNSUPPORTED = 0, 3
+
+
+def range_bytes(block_step, bm_range, radius, ps_range):
+    """Shared memory of the one-warp CTA by which a range is accepted or refused."""
+    ws, wt, reach = 2 * bm_range + 1, 2 * ps_range + 1, bm_range + radius * ps_range
+
+    def over(w, k):
+        return -(-w // k) * k - w
+
+    def cost(k):
+        total = 0.0
+        for w, n in ((ws, ws * ws), (wt, 4.0 * radius * wt * wt)):
+            total += n * (w + over(w, k)) / w * (143.0 + 8.0 * (k + 7) / k)
+        return total
+
+    k = min(range(8, 13), key=cost)
+    extra = max(over(ws, k), over(wt, k) if radius else 0)
+    pitch = 3 * block_step + 2 * reach + 16 + extra
+    return 4 * pitch * (7 * block_step + 2 * reach + 8) + 1024
+
+
+@pytest.mark.parametrize("block_step", range(1, 9))
+def test_accepted_searches_fit(engine_lib, block_step):
+    lanes, shared, limit = ctypes.c_int(), ctypes.c_longlong(), ctypes.c_longlong()
+    forms, refused = set(), 0
+    bm_ranges = [*range(1, 8), *range(8, 80, 6), *range(80, 116)]
+    for radius, ps_num, ps_range in [(0, 2, 4), (1, 2, 1), (1, 2, 6), (1, 3, 6), (2, 1, 4),
+                                     (2, 2, 6), (3, 8, 9), (7, 2, 3)]:
+        for bm_range in bm_ranges:
+            for w, h, windows in [(8, 8, 1), (300, 169, 1), (640, 360, 1), (960, 540, 2),
+                                  (1920, 1080, 30)]:
+                rc = engine_lib.bm3d_b200_selftest_match_plan(
+                    w, h, block_step, bm_range, radius, ps_num, ps_range, windows,
+                    ctypes.byref(lanes), ctypes.byref(shared), ctypes.byref(limit))
+                case = (block_step, bm_range, radius, ps_num, ps_range, w, h, windows)
+                if range_bytes(block_step, bm_range, radius, ps_range) > 220 * 1024:
+                    assert rc == UNSUPPORTED, case
+                    refused += 1
+                    continue
+                assert rc == OK, case
+                assert limit.value == 227 * 1024
+                assert shared.value <= limit.value, (case, lanes.value, shared.value)
+                forms.add(lanes.value)
+    assert {1, 8} <= forms and refused

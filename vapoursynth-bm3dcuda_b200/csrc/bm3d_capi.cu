@@ -2691,3 +2691,20 @@ extern "C" int bm3d_b200_selftest_reciprocal(unsigned lo_bits, unsigned hi_bits,
     if (first_bad) *first_bad = first;
     return BM3D_B200_OK;
 }
+
+extern "C" int bm3d_b200_selftest_match_plan(int width, int height, int block_step, int bm_range,
+                                             int radius, int ps_num, int ps_range, int windows,
+                                             int *lanes, long long *shared_bytes,
+                                             long long *limit_bytes) {
+    if (!lanes || !shared_bytes || !limit_bytes || windows < 1)
+        return fail(BM3D_B200_ERR_INVALID, "selftest: invalid arguments");
+    if (int rc = check_search(width, height, width, block_step, bm_range, radius, ps_num,
+                              ps_range))
+        return rc;
+    const MatchGeometry g =
+        match_geometry(width, height, block_step, bm_range, radius, ps_num, ps_range);
+    *lanes = match_lanes(g, radius, windows);
+    *shared_bytes = (long long)(*lanes == 1 ? g.smem : g.split[*lanes == 4 ? 0 : 1].smem);
+    *limit_bytes = (long long)kMatchSmemMax;
+    return BM3D_B200_OK;
+}

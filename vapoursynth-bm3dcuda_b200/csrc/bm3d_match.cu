@@ -133,8 +133,12 @@ void choose_pitches(MatchGeometry &g, int block_step, int bm_range, int radius, 
         auto &sp = g.split[i];
         const int tw = (4 * kSplitWx - 1) * block_step + 2 * mmax + 8 + g.extra_cols;
         sp.tile_rows = (kSplitWy * 8 / lanes - 1) * block_step + 2 * mmax + 8;
+        const auto bytes = [&](int pitch) {
+            return (size_t)pitch * sp.tile_rows * sizeof(float) + lists * kSplitWx * kSplitWy;
+        };
         sp.pitch = pick_pitch(tw + 8, block_step, 2 + i);
-        sp.smem = (size_t)sp.pitch * sp.tile_rows * sizeof(float) + lists * kSplitWx * kSplitWy;
+        if (bytes(sp.pitch) > kMatchSmemMax) sp.pitch = tw + 8;
+        sp.smem = bytes(sp.pitch);
     }
 }
 
@@ -207,8 +211,6 @@ long long match_tiles(const MatchGeometry &g, int nwin) {
     return (long long)((g.nbx + 4 * g.wx - 1) / (4 * g.wx)) * ((g.nby + 7) / 8) * nwin;
 }
 
-namespace {
-
 // Lanes per reference block: one, unless the launch leaves most of the GPU's
 // 148 x 12 resident warps idle, or the search range lets an SM hold only one
 // CTA of four warps with one lane per block (the split tiles hold 32 blocks, not
@@ -224,15 +226,16 @@ namespace {
 //   960 warps (8 x 640x360, r 0)       95  107  123
 //   one CTA per SM: 2 x 1920x1080, r 3, bm_range 16, ps_range 6   1839  1724
 //                   2 x 1280x720, r 2, bm_range 20, ps_range 8    1046   923
-int match_lanes(const MatchParams &p, const MatchGeometry &g, int nwin) {
+// Ranges near the limit fit the one-warp CTA of one lane per block but not the
+// four-warp CTA of the split forms.
+int match_lanes(const MatchGeometry &g, int radius, int nwin) {
     const long long warps =
-        (long long)((p.nbx + 3) / 4) * ((p.nby + 7) / 8) * nwin;  // of 4 x 8 blocks
-    if (warps <= 160) return 8;
-    if (warps <= (p.radius == 0 ? 600 : 450)) return 4;
+        (long long)((g.nbx + 3) / 4) * ((g.nby + 7) / 8) * nwin;  // of 4 x 8 blocks
+    const bool fits[2] = {g.split[0].smem <= kMatchSmemMax, g.split[1].smem <= kMatchSmemMax};
+    if (warps <= 160 && fits[1]) return 8;
+    if (warps <= (radius == 0 ? 600 : 450) && fits[0]) return 4;
     return kSmemPerSm / (g.smem + 1024) * g.wx <= 4 && g.split[0].smem < g.smem / 2 ? 4 : 1;
 }
-
-}  // namespace
 
 cudaError_t launch_match_split(const MatchParams &p, const MatchGeometry &g, int nwin, int lanes,
                                cudaStream_t stream) {
@@ -248,7 +251,7 @@ cudaError_t launch_match_split(const MatchParams &p, const MatchGeometry &g, int
 
 cudaError_t launch_match(const MatchParams &p, const MatchGeometry &g, int nwin,
                          cudaStream_t stream) {
-    const int lanes = match_lanes(p, g, nwin);
+    const int lanes = match_lanes(g, p.radius, nwin);
     if (p.metric != 0) {
         const int ws = 2 * p.bm_range + 1, wt = 2 * p.ps_range + 1;
         const double spatial = (double)ws * ws, temporal = 2.0 * p.radius * p.ps_num * wt * wt;
