@@ -562,6 +562,12 @@ BM3D_B200_API int bm3d_b200_selftest_match_plan(int width, int height, int block
                                                 int bm_range, int radius, int ps_num,
                                                 int ps_range, int windows, int *lanes,
                                                 long long *shared_bytes, long long *limit_bytes);
+/* The same for the matching CTAs of a batch that holds one such clip, with
+ * `cta_warps` warps (1, 2, 4) and strips of `strip` candidates (8 .. 12). */
+BM3D_B200_API int bm3d_b200_selftest_batch_plan(int width, int height, int block_step,
+                                                int bm_range, int radius, int ps_num,
+                                                int ps_range, int cta_warps, int strip,
+                                                long long *shared_bytes, long long *limit_bytes);
 
 #ifdef __cplusplus
 }

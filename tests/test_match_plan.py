@@ -8,8 +8,9 @@ import pytest
 OK, UNSUPPORTED = 0, 3
 
 
-def range_bytes(block_step, bm_range, radius, ps_range):
-    """Shared memory of the one-warp CTA by which a range is accepted or refused."""
+def range_bytes(block_step, bm_range, radius, ps_range, warps=1, strip=None):
+    """Shared memory of the CTA (one warp for single launches) by which a range is
+    accepted or refused."""
     ws, wt, reach = 2 * bm_range + 1, 2 * ps_range + 1, bm_range + radius * ps_range
 
     def over(w, k):
@@ -21,10 +22,10 @@ def range_bytes(block_step, bm_range, radius, ps_range):
             total += n * (w + over(w, k)) / w * (143.0 + 8.0 * (k + 7) / k)
         return total
 
-    k = min(range(8, 13), key=cost)
+    k = strip or min(range(8, 13), key=cost)
     extra = max(over(ws, k), over(wt, k) if radius else 0)
-    pitch = 3 * block_step + 2 * reach + 16 + extra
-    return 4 * pitch * (7 * block_step + 2 * reach + 8) + 1024
+    pitch = (4 * warps - 1) * block_step + 2 * reach + 16 + extra
+    return 4 * pitch * (7 * block_step + 2 * reach + 8) + 1024 * warps
 
 
 @pytest.mark.parametrize("block_step", range(1, 9))
@@ -50,3 +51,21 @@ def test_accepted_searches_fit(engine_lib, block_step):
                 assert shared.value <= limit.value, (case, lanes.value, shared.value)
                 forms.add(lanes.value)
     assert {1, 8} <= forms and refused
+
+
+@pytest.mark.parametrize("block_step", range(1, 9))
+def test_accepted_batches_fit(engine_lib, block_step):
+    shared, limit = ctypes.c_longlong(), ctypes.c_longlong()
+    for radius, ps_num, ps_range in [(0, 2, 4), (1, 2, 1), (1, 2, 6), (1, 3, 6), (2, 2, 4),
+                                     (2, 2, 6), (3, 8, 9)]:
+        for bm_range in range(20, 116):
+            for warps in (1, 2, 4):
+                for strip in range(8, 13):
+                    rc = engine_lib.bm3d_b200_selftest_batch_plan(
+                        640, 360, block_step, bm_range, radius, ps_num, ps_range, warps, strip,
+                        ctypes.byref(shared), ctypes.byref(limit))
+                    case = (block_step, bm_range, radius, ps_num, ps_range, warps, strip)
+                    need = range_bytes(block_step, bm_range, radius, ps_range, warps, strip)
+                    assert rc == (UNSUPPORTED if need > 220 * 1024 else OK), case
+                    if rc == OK:
+                        assert shared.value <= limit.value == 227 * 1024, (case, shared.value)

@@ -152,7 +152,21 @@ void choose_match_form(bm3d_b200_batch *b) {
     }
     b->kt = work[1] > work[0] ? 11 : 9;
     for (const BatchClip &c : b->clips)
-        b->small &= clip_geometry(b, c).smem <= kMatchSmemMax;
+        b->small &= clip_geometry(b, c).smem <= kMatchBatchSmemMax;
+}
+
+// Matching geometry of clip i in the batch's form.
+int clip_match_geometry(const bm3d_b200_batch *b, int i, MatchGeometry *g) {
+    const BatchClip &c = b->clips[i];
+    const bm3d_b200_params &p = c.prm;
+    const size_t range_bytes = match_range_bytes(p.block_step[0], p.bm_range[0], p.radius,
+                                                 p.ps_range[0], b->wx, b->K);
+    if (range_bytes > kMatchSmemLimit)
+        return bfail(BM3D_B200_ERR_UNSUPPORTED, "BM3D batch: clip %d needs %zu B of shared memory",
+                     i, range_bytes);
+    *g = clip_geometry(b, c);
+    choose_pitches(*g, p.block_step[0], p.bm_range[0], p.radius, p.ps_range[0], kMatchBatchSmemMax);
+    return BM3D_B200_OK;
 }
 
 // Stage tables of one clip (fused VAggregate mapping, source/source.cpp:830-844).
@@ -203,14 +217,8 @@ int prepare(bm3d_b200_batch *b) {
         BatchClip &c = b->clips[i];
         const int N = c.n, tw = 2 * c.prm.radius + 1;
         const size_t ntab = (size_t)N * tw, plane = (size_t)c.h * c.stride;
-        MatchGeometry g = clip_geometry(b, c);
-        choose_pitches(g, c.prm.block_step[0], c.prm.bm_range[0], c.prm.radius, c.prm.ps_range[0]);
-        const size_t range_bytes =
-            match_range_bytes(c.prm.block_step[0], c.prm.bm_range[0], c.prm.radius,
-                              c.prm.ps_range[0], b->wx, b->K);
-        if (range_bytes > kMatchSmemLimit)
-            return bfail(BM3D_B200_ERR_UNSUPPORTED, "BM3D batch: clip %d needs %zu B of shared memory",
-                         i, range_bytes);
+        MatchGeometry g;
+        if (int rc = clip_match_geometry(b, i, &g)) return rc;
         b->match_smem = std::max(b->match_smem, g.smem);
         if (!c.d_basic) {
             BTRY(cudaMalloc(&c.d_basic, (size_t)N * plane * sizeof(float)));
@@ -589,4 +597,33 @@ extern "C" void bm3d_b200_batch_destroy(bm3d_b200_batch *b) {
     for (auto &c : b->clips) release_clip_scratch(c);
     if (b->cap) cudaStreamDestroy(b->cap);
     delete b;
+}
+
+extern "C" int bm3d_b200_selftest_batch_plan(int width, int height, int block_step, int bm_range,
+                                             int radius, int ps_num, int ps_range, int cta_warps,
+                                             int strip, long long *shared_bytes,
+                                             long long *limit_bytes) {
+    if (!shared_bytes || !limit_bytes || width < 8 || height < 8 || block_step < 1 ||
+        block_step > 8 || bm_range < 1 || radius < 0 || ps_num < 1 || ps_num > 8 || ps_range < 1 ||
+        (cta_warps != 1 && cta_warps != 2 && cta_warps != 4) || strip < 8 || strip > 12)
+        return bfail(BM3D_B200_ERR_INVALID, "selftest: invalid arguments");
+    bm3d_b200_batch b;
+    BatchClip c;
+    c.w = width;
+    c.h = height;
+    c.n = 1;
+    c.prm.block_step[0] = block_step;
+    c.prm.bm_range[0] = bm_range;
+    c.prm.radius = radius;
+    c.prm.ps_num[0] = ps_num;
+    c.prm.ps_range[0] = ps_range;
+    b.clips.push_back(c);
+    b.wx = cta_warps;
+    b.K = strip;
+    choose_match_form(&b);
+    MatchGeometry g;
+    if (int rc = clip_match_geometry(&b, 0, &g)) return rc;
+    *shared_bytes = (long long)(g.smem + kMatchBatchStatic);
+    *limit_bytes = (long long)kMatchSmemMax;
+    return BM3D_B200_OK;
 }

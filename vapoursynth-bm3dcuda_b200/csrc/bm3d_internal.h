@@ -56,8 +56,11 @@ struct MatchParams {
 
 // Search ranges whose one-warp CTA needs more shared memory are refused.
 constexpr size_t kMatchSmemLimit = 220 * 1024;
-// Largest dynamic shared memory of a matching launch.
+// Largest shared memory of a matching CTA, and what the batch kernel's own
+// variables take of it.
 constexpr size_t kMatchSmemMax = 227 * 1024;
+constexpr size_t kMatchBatchStatic = 256;
+constexpr size_t kMatchBatchSmemMax = kMatchSmemMax - kMatchBatchStatic;
 
 struct MatchGeometry {
     int nbx, nby;
@@ -84,8 +87,10 @@ size_t match_range_bytes(int block_step, int bm_range, int radius, int ps_range,
 // Geometry with a given CTA width (warps) and strip widths (autotuner).
 MatchGeometry match_geometry_with(int width, int height, int block_step, int bm_range, int radius,
                                   int ps_range, int wx, int ks, int kt, bool small);
-// Its shared-memory row pitches, and the tiles of the split launches.
-void choose_pitches(MatchGeometry &g, int block_step, int bm_range, int radius, int ps_range);
+// Its shared-memory row pitches, for CTAs of up to `limit` bytes, and the tiles of
+// the split launches.
+void choose_pitches(MatchGeometry &g, int block_step, int bm_range, int radius, int ps_range,
+                    size_t limit = kMatchSmemMax);
 // Strip width of the temporal windows (small geometries).
 int temporal_strip_width(int ps_range);
 // Resident CTAs per SM (2 or 3) that a launch of the small search aims at.

@@ -114,7 +114,8 @@ MatchGeometry match_geometry_with(int width, int height, int block_step, int bm_
     return g;
 }
 
-void choose_pitches(MatchGeometry &g, int block_step, int bm_range, int radius, int ps_range) {
+void choose_pitches(MatchGeometry &g, int block_step, int bm_range, int radius, int ps_range,
+                    size_t limit) {
     const int mmax = bm_range + radius * ps_range;
     const size_t lists = g.small ? kSmallListBytes : kListBytes;
     // the conflict-free pitch where it costs no resident CTA (block steps 4 and
@@ -124,7 +125,7 @@ void choose_pitches(MatchGeometry &g, int block_step, int bm_range, int radius, 
     const auto resident = [&](size_t bytes) {
         return std::min<size_t>(12 / g.wx, kSmemPerSm / (bytes + 1024));
     };
-    if (smem <= kMatchSmemMax && resident(smem) == resident(g.smem)) {
+    if (smem <= limit && resident(smem) == resident(g.smem)) {
         g.pitch = pitch;
         g.smem = smem;
     }

@@ -15,6 +15,7 @@ __global__ void __launch_bounds__(128, CTAS) match_batch_kernel(MatchBatch b) {
     extern __shared__ float tile[];
     __shared__ MatchParams ps;
     __shared__ long long item_s;
+    static_assert(sizeof(ps) + sizeof(item_s) <= kMatchBatchStatic, "room beside the tile");
     const long long total = b.item_off[b.nclips];
     const int nbx_cta = (blockDim.x >> 5) * 4;
     for (;;) {
@@ -74,7 +75,7 @@ cudaError_t launch_match_batch_k(const MatchBatch &b, int kt, bool small, int wx
 
 cudaError_t launch_match_batch(const MatchBatch &b, int K, int kt, bool small, int wx, size_t smem,
                                cudaStream_t stream) {
-    if (smem > kMatchSmemMax) return cudaErrorInvalidValue;
+    if (smem > kMatchBatchSmemMax) return cudaErrorInvalidValue;
     switch (K) {
         case 9: return launch_match_batch_k<9>(b, kt, small, wx, smem, stream);
         case 10: return launch_match_batch_k<10>(b, kt, small, wx, smem, stream);
