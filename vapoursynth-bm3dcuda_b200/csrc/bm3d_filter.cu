@@ -725,6 +725,8 @@ __global__ void __launch_bounds__(128, filter_ctas_per_sm<FINAL, TC, VAR, SC>())
 
 // Persistent form over a batch of clips: resident CTAs take CTA-sized group
 // ranges from a shared counter, clip-major. TMA: every clip has a tensor map.
+// The maps lie in global memory, where another batch's may have been before, so a
+// CTA that moves to a clip first orders its copy with the reads of the TMA unit.
 template <bool FINAL, bool TMA>
 __global__ void __launch_bounds__(128, filter_ctas_per_sm<FINAL, false, false, kScatterBoxes>())
     filter_batch_kernel(FilterBatch b) {
@@ -732,6 +734,7 @@ __global__ void __launch_bounds__(128, filter_ctas_per_sm<FINAL, false, false, k
     __shared__ FilterParams ps;
     __shared__ long long item_s;
     const long long total = b.item_off[b.nclips];
+    int clip = -1;
     for (;;) {
         if (threadIdx.x == 0) item_s = (long long)atomicAdd(b.counter, 1ULL);
         __syncthreads();
@@ -743,9 +746,14 @@ __global__ void __launch_bounds__(128, filter_ctas_per_sm<FINAL, false, false, k
             if (b.item_off[mid] <= item) lo = mid; else hi = mid;
         }
         if (threadIdx.x == 0) ps = b.clips[lo];
+        if (TMA && lo != clip) {
+            asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(b.maps + lo)
+                         : "memory");
+            clip = lo;
+        }
         __syncthreads();
-        filter_cta<FINAL, false, false, TMA ? kScatterBoxes : kScatterLsu>(ps, TMA ? b.maps + lo : nullptr,
-                                             item - b.item_off[lo], fsm);
+        filter_cta<FINAL, false, false, TMA ? kScatterBoxes : kScatterLsu>(
+            ps, TMA ? b.maps + lo : nullptr, item - b.item_off[lo], fsm);
         __syncthreads();
     }
 }
