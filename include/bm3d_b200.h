@@ -568,6 +568,10 @@ BM3D_B200_API int bm3d_b200_selftest_batch_plan(int width, int height, int block
                                                 int bm_range, int radius, int ps_num,
                                                 int ps_range, int cta_warps, int strip,
                                                 long long *shared_bytes, long long *limit_bytes);
+/* Candidates per strip of a search with one of the run-time-compiled plugin's
+ * distances other than SSD. */
+BM3D_B200_API int bm3d_b200_selftest_metric_strip(int bm_range, int radius, int ps_num,
+                                                  int ps_range);
 
 #ifdef __cplusplus
 }

@@ -69,3 +69,18 @@ def test_accepted_batches_fit(engine_lib, block_step):
                     assert rc == (UNSUPPORTED if need > 220 * 1024 else OK), case
                     if rc == OK:
                         assert shared.value <= limit.value == 227 * 1024, (case, shared.value)
+
+
+def test_strips_suit_narrow_windows(engine_lib):
+    """The run-time-compiled plugin's distances: no search computes its candidates
+    2.25 times (strips of 8 over windows of 3 columns would compute 2.67 times)."""
+    for bm_range in range(1, 41):
+        for radius in range(4):
+            for ps_num in range(1, 9):
+                for ps_range in range(1, 11):
+                    k = engine_lib.bm3d_b200_selftest_metric_strip(bm_range, radius, ps_num,
+                                                                   ps_range)
+                    windows = [(1, 2 * bm_range + 1), (2 * radius * ps_num, 2 * ps_range + 1)]
+                    computed = sum(n * w * -(-w // k) * k for n, w in windows)
+                    assert computed < 2.25 * sum(n * w * w for n, w in windows), (
+                        bm_range, radius, ps_num, ps_range, k)

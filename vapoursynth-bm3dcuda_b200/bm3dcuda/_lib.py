@@ -82,6 +82,7 @@ SIGNATURES = {
     "bm3d_b200_selftest_match_plan": (c_int, [c_int] * 8 + [ctypes.POINTER(c_int),
                                                             ctypes.POINTER(c_ll),
                                                             ctypes.POINTER(c_ll)]),
+    "bm3d_b200_selftest_metric_strip": (c_int, [c_int] * 4),
     "bm3d_b200_selftest_batch_plan": (c_int, [c_int] * 9 + [ctypes.POINTER(c_ll)] * 2),
     "bm3d_b200_batch_create": (c_int, [ctypes.POINTER(c_void_p), c_int]),
     "bm3d_b200_batch_add": (c_int, [c_void_p, c_int, c_int, c_int, ctypes.POINTER(Params),

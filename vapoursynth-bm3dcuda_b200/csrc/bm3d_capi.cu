@@ -2708,3 +2708,8 @@ extern "C" int bm3d_b200_selftest_match_plan(int width, int height, int block_st
     *limit_bytes = (long long)kMatchSmemMax;
     return BM3D_B200_OK;
 }
+
+extern "C" int bm3d_b200_selftest_metric_strip(int bm_range, int radius, int ps_num,
+                                               int ps_range) {
+    return metric_strip_width(bm_range, radius, ps_num, ps_range);
+}

@@ -91,6 +91,13 @@ MatchGeometry match_geometry_with(int width, int height, int block_step, int bm_
 // the split launches.
 void choose_pitches(MatchGeometry &g, int block_step, int bm_range, int radius, int ps_range,
                     size_t limit = kMatchSmemMax);
+// A shared-memory row pitch for CTA tiles of tile_rows rows and list_bytes: of at
+// least `base` words, with the fewest bank conflicts, but `base` where that saves no
+// factor of `gain`, exceeds `limit` or lets fewer than `ctas` CTAs share an SM that could.
+int match_pitch(int base, int block_step, int log_lanes, int tile_rows, size_t list_bytes,
+                int ctas, size_t limit, double gain = 1.0);
+// Strip width (4, 8, 10) of the searches with p.metric != 0.
+int metric_strip_width(int bm_range, int radius, int ps_num, int ps_range);
 // Strip width of the temporal windows (small geometries).
 int temporal_strip_width(int ps_range);
 // Resident CTAs per SM (2 or 3) that a launch of the small search aims at.
@@ -107,7 +114,7 @@ cudaError_t launch_match_split(const MatchParams &p, const MatchGeometry &g, int
                                cudaStream_t stream);
 cudaError_t launch_match_pairs(const MatchParams &p, const MatchGeometry &g, int nwin, int lanes,
                                cudaStream_t stream);
-// launch_match for p.metric != 0, in strips of K (8, 10), with 1 or 4 lanes per block.
+// launch_match for p.metric != 0, in strips of K (4, 8, 10), with 1 or 4 lanes per block.
 cudaError_t launch_match_metric(const MatchParams &p, const MatchGeometry &g, int nwin, int K,
                                 int lanes, cudaStream_t stream);
 

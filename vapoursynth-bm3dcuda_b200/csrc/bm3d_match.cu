@@ -47,12 +47,12 @@ int choose_strip_width(int w, const int (&widths)[N]) {
 // conflicts when all lanes read the same candidate offset, summed over the 8
 // phases of the row skew. It runs with each call that plans its own search, so
 // it counts bank masks instead of lanes (1.0 us for a pitch, 5.3 lane by
-// lane).
-int pick_pitch(int base, int block_step, int log_lanes) {
+// lane). `gain`: a pitch has to save that factor of the base's conflicts.
+int pick_pitch(int base, int block_step, int log_lanes, double gain) {
     const int rows = 8 >> log_lanes, lanes = 1 << log_lanes;
     // the banks of four neighbouring blocks, distinct for every block_step up to 8
     const unsigned quad = 1u | 1u << block_step | 1u << 2 * block_step | 1u << 3 * block_step;
-    int best = base, best_cost = 1 << 30;
+    int best = base, best_cost = 1 << 30, base_cost = 0;
     for (int pitch = base; pitch < base + 16 && best_cost > 8; ++pitch) {
         int cost = 0;
         // a phase costs at least 1: stop where the pitch cannot win any more
@@ -73,12 +73,13 @@ int pick_pitch(int base, int block_step, int log_lanes) {
             for (int k = 0; k < 8 && hit[k]; ++k) ++cost;
             if (phase < 7 && cost + 7 - phase >= best_cost) cost = best_cost;
         }
+        if (pitch == base) base_cost = cost;
         if (cost < best_cost) {
             best_cost = cost;
             best = pitch;
         }
     }
-    return best;
+    return best_cost * gain > base_cost ? base : best;
 }
 
 // A warp's match lists: 16 words per thread (SMALL), else 8.
@@ -87,6 +88,40 @@ constexpr size_t kSmallListBytes = 16 * 32 * sizeof(int), kListBytes = 8 * 32 * 
 constexpr size_t kSmemPerSm = 228 * 1024;
 
 }  // namespace
+
+int match_pitch(int base, int block_step, int log_lanes, int tile_rows, size_t list_bytes,
+                int ctas, size_t limit, double gain) {
+    const int pitch = pick_pitch(base, block_step, log_lanes, gain);
+    const auto bytes = [&](int p) { return (size_t)p * tile_rows * sizeof(float) + list_bytes; };
+    const auto resident = [&](int p) {
+        return std::min<size_t>(ctas, kSmemPerSm / (bytes(p) + 1024));
+    };
+    return bytes(pitch) <= limit && resident(pitch) == resident(base) ? pitch : base;
+}
+
+// 8 or 10 as for the SSD; 4 where that spares a third of the candidates computed
+// (the list costs more in narrow strips: windows of 11 columns run 4% faster in
+// strips of 4 than of 8 in the spatial stage, up to 8% slower in the temporal ones).
+// Whole-window time with strips of 4 / 8 / 10 against one candidate at a time, ZSSD,
+// 1320x428 at block_step 2:
+//   bm_range 1, radius 0                           0.87 0.91 0.93
+//   bm_range 5, radius 1, ps_num 2, ps_range 1     0.72 0.83 0.92
+//   bm_range 6, radius 0                           0.77 0.72 0.80
+//   bm_range 9, radius 0                           0.52 0.53 0.47
+//   bm_range 4, radius 1, ps_num 8, ps_range 1     0.86 1.08 1.12
+//   bm_range 9, radius 1, ps_num 4, ps_range 4     0.82 0.83 0.58
+int metric_strip_width(int bm_range, int radius, int ps_num, int ps_range) {
+    const int ws = 2 * bm_range + 1, wt = 2 * ps_range + 1;
+    const double spatial = (double)ws * ws, temporal = 2.0 * radius * ps_num * wt * wt;
+    const auto cost = [&](int K) {
+        return spatial * strip_cost(ws, K) + temporal * strip_cost(wt, K);
+    };
+    const auto computed = [&](int K) {
+        return spatial * ((ws + K - 1) / K * K) / ws + temporal * ((wt + K - 1) / K * K) / wt;
+    };
+    const int K = cost(10) < cost(8) ? 10 : 8;
+    return 1.5 * computed(4) <= computed(K) ? 4 : K;
+}
 
 int temporal_strip_width(int ps_range) {
     const int widths[] = {8, 9, 11};
@@ -120,26 +155,16 @@ void choose_pitches(MatchGeometry &g, int block_step, int bm_range, int radius, 
     const size_t lists = g.small ? kSmallListBytes : kListBytes;
     // the conflict-free pitch where it costs no resident CTA (block steps 4 and
     // 2 meet 4-way bank conflicts at an arbitrary pitch)
-    const int pitch = pick_pitch(g.pitch, block_step, 0);
-    const size_t smem = (size_t)pitch * g.tile_rows * sizeof(float) + lists * g.wx;
-    const auto resident = [&](size_t bytes) {
-        return std::min<size_t>(12 / g.wx, kSmemPerSm / (bytes + 1024));
-    };
-    if (smem <= limit && resident(smem) == resident(g.smem)) {
-        g.pitch = pitch;
-        g.smem = smem;
-    }
+    g.pitch = match_pitch(g.pitch, block_step, 0, g.tile_rows, lists * g.wx, 12 / g.wx, limit);
+    g.smem = (size_t)g.pitch * g.tile_rows * sizeof(float) + lists * g.wx;
     for (int i = 0; i < 2; ++i) {
         const int lanes = 4 << i;
         auto &sp = g.split[i];
         const int tw = (4 * kSplitWx - 1) * block_step + 2 * mmax + 8 + g.extra_cols;
         sp.tile_rows = (kSplitWy * 8 / lanes - 1) * block_step + 2 * mmax + 8;
-        const auto bytes = [&](int pitch) {
-            return (size_t)pitch * sp.tile_rows * sizeof(float) + lists * kSplitWx * kSplitWy;
-        };
-        sp.pitch = pick_pitch(tw + 8, block_step, 2 + i);
-        if (bytes(sp.pitch) > kMatchSmemMax) sp.pitch = tw + 8;
-        sp.smem = bytes(sp.pitch);
+        sp.pitch = match_pitch(tw + 8, block_step, 2 + i, sp.tile_rows,
+                               lists * kSplitWx * kSplitWy, 1, kMatchSmemMax);
+        sp.smem = (size_t)sp.pitch * sp.tile_rows * sizeof(float) + lists * kSplitWx * kSplitWy;
     }
 }
 
@@ -254,13 +279,8 @@ cudaError_t launch_match(const MatchParams &p, const MatchGeometry &g, int nwin,
                          cudaStream_t stream) {
     const int lanes = match_lanes(g, p.radius, nwin);
     if (p.metric != 0) {
-        const int ws = 2 * p.bm_range + 1, wt = 2 * p.ps_range + 1;
-        const double spatial = (double)ws * ws, temporal = 2.0 * p.radius * p.ps_num * wt * wt;
-        auto cost = [&](int K) {
-            return spatial * strip_cost(ws, K) + temporal * strip_cost(wt, K);
-        };
-        return launch_match_metric(p, g, nwin, cost(10) < cost(8) ? 10 : 8, lanes == 1 ? 1 : 4,
-                                   stream);
+        const int K = metric_strip_width(p.bm_range, p.radius, p.ps_num, p.ps_range);
+        return launch_match_metric(p, g, nwin, K, lanes == 1 ? 1 : 4, stream);
     }
     return launch_match_split(p, g, nwin, lanes, stream);
 }

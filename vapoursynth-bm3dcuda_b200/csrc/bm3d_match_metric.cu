@@ -19,12 +19,19 @@ cudaError_t launch_metric(MatchParams q, const MatchGeometry &g, int nwin, int l
     const int rows = 8 / lanes * wy;  // block rows of a CTA
     q.pitch = (4 * wx - 1) * q.block_step + 2 * mmax + 16 + q.extra_cols;
     q.tile_rows = (rows - 1) * q.block_step + 2 * mmax + 8;
-    const size_t smem = (size_t)q.pitch * q.tile_rows * sizeof(float) +
-                        (size_t)(SMALL ? 16 : 8) * 32 * wx * wy * sizeof(int);
+    const size_t lists = (size_t)(SMALL ? 16 : 8) * 32 * wx * wy * sizeof(int);
+    const auto bytes = [&] { return (size_t)q.pitch * q.tile_rows * sizeof(float) + lists; };
     // a range that only just fits: one candidate per strip needs no extra columns
-    if (smem > kMatchSmemMax)
+    if (bytes() > kMatchSmemMax)
         return K == 1 ? cudaErrorInvalidValue
                       : launch_metric<1, M, false>(q, g, nwin, 1, stream);
+    // Another pitch where the base one meets clearly more conflicts (it has 18 in 8
+    // accesses at block_step 3 and 7, where 16 gain nothing: 158x501, ps_num 3: 529 us,
+    // 557 at the other; 900x300 at block_step 1, bm_range 9, radius 1, ps_num 4,
+    // 64 in 8: 9.26 ms in strips of 8, 4.49 with 15 in 8, 3.18 in strips of 10).
+    q.pitch = match_pitch(q.pitch, q.block_step, lanes == 1 ? 0 : 2, q.tile_rows, lists,
+                          12 / (wx * wy), kMatchSmemMax, 1.5);
+    const size_t smem = bytes();
     const dim3 grid((q.nbx + 4 * wx - 1) / (4 * wx), (q.nby + rows - 1) / rows, nwin);
     const dim3 block(32 * wx * wy);
     if constexpr (SMALL) {
@@ -37,12 +44,21 @@ cudaError_t launch_metric(MatchParams q, const MatchGeometry &g, int nwin, int l
     return launch_match_t<K, K, M, 1, SMALL>(q, grid, block, smem, stream);
 }
 
+template <int K, int M>
+cudaError_t launch_metric_k(const MatchParams &p, const MatchGeometry &g, int nwin, int lanes,
+                            cudaStream_t stream) {
+    return p.radius > 0 && p.ps_num > 2 ? launch_metric<K, M, false>(p, g, nwin, 1, stream)
+                                        : launch_metric<K, M, true>(p, g, nwin, lanes, stream);
+}
+
 template <int M>
 cudaError_t launch_metric_m(const MatchParams &p, const MatchGeometry &g, int nwin, int K,
                             int lanes, cudaStream_t stream) {
-    if (p.radius > 0 && p.ps_num > 2) return launch_metric<8, M, false>(p, g, nwin, 1, stream);
-    return K == 10 ? launch_metric<10, M, true>(p, g, nwin, lanes, stream)
-                   : launch_metric<8, M, true>(p, g, nwin, lanes, stream);
+    switch (K) {
+        case 4: return launch_metric_k<4, M>(p, g, nwin, lanes, stream);
+        case 10: return launch_metric_k<10, M>(p, g, nwin, lanes, stream);
+        default: return launch_metric_k<8, M>(p, g, nwin, lanes, stream);
+    }
 }
 
 }  // namespace
