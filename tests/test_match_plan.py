@@ -84,3 +84,16 @@ def test_strips_suit_narrow_windows(engine_lib):
                     computed = sum(n * w * -(-w // k) * k for n, w in windows)
                     assert computed < 2.25 * sum(n * w * w for n, w in windows), (
                         bm_range, radius, ps_num, ps_range, k)
+
+
+def test_small_windows_are_not_shared(engine_lib):
+    """Several lanes per block scan a window of 25 candidates slower than one, once
+    a launch has a few warps for every SM."""
+    lanes, shared, limit = ctypes.c_int(), ctypes.c_longlong(), ctypes.c_longlong()
+    for w, h, step, bm_range, want in [(640, 360, 8, 2, 8), (960, 540, 8, 2, 4),
+                                       (1280, 720, 8, 2, 1), (1280, 720, 8, 1, 1),
+                                       (700, 400, 4, 2, 1), (1280, 720, 8, 9, 4)]:
+        assert engine_lib.bm3d_b200_selftest_match_plan(
+            w, h, step, bm_range, 0, 2, 4, 1, ctypes.byref(lanes), ctypes.byref(shared),
+            ctypes.byref(limit)) == OK
+        assert lanes.value == want, (w, h, step, bm_range, lanes.value)

@@ -2703,7 +2703,7 @@ extern "C" int bm3d_b200_selftest_match_plan(int width, int height, int block_st
         return rc;
     const MatchGeometry g =
         match_geometry(width, height, block_step, bm_range, radius, ps_num, ps_range);
-    *lanes = match_lanes(g, radius, windows);
+    *lanes = match_lanes(g, bm_range, radius, windows);
     *shared_bytes = (long long)(*lanes == 1 ? g.smem : g.split[*lanes == 4 ? 0 : 1].smem);
     *limit_bytes = (long long)kMatchSmemMax;
     return BM3D_B200_OK;

@@ -103,7 +103,7 @@ int temporal_strip_width(int ps_range);
 // Resident CTAs per SM (2 or 3) that a launch of the small search aims at.
 int match_ctas(const MatchGeometry &g, int nwin);
 // Lanes per reference block (1, 4, 8) of a launch over nwin windows.
-int match_lanes(const MatchGeometry &g, int radius, int nwin);
+int match_lanes(const MatchGeometry &g, int bm_range, int radius, int nwin);
 // CTA tiles of one launch over nwin windows.
 long long match_tiles(const MatchGeometry &g, int nwin);
 cudaError_t launch_match(const MatchParams &p, const MatchGeometry &g, int nwin,

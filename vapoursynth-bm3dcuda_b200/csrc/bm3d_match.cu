@@ -252,14 +252,21 @@ long long match_tiles(const MatchGeometry &g, int nwin) {
 //   960 warps (8 x 640x360, r 0)       95  107  123
 //   one CTA per SM: 2 x 1920x1080, r 3, bm_range 16, ps_range 6   1839  1724
 //                   2 x 1280x720, r 2, bm_range 20, ps_range 8    1046   923
+// Windows of 5 x 5 and less are little work to share (bm_range 2, radius 0):
+//   200 warps (800x450)              16.6 13.0 14.7
+//   270 warps (960x540)              16.9 13.6 15.6
+//   350 warps (1100x620)             17.0 18.5 18.8
+//   480 warps (1280x720)             16.6 19.5 22.8
+//   572 warps (700x400 step 4)       16.1 20.3 25.0
 // Ranges near the limit fit the one-warp CTA of one lane per block but not the
 // four-warp CTA of the split forms.
-int match_lanes(const MatchGeometry &g, int radius, int nwin) {
+int match_lanes(const MatchGeometry &g, int bm_range, int radius, int nwin) {
     const long long warps =
         (long long)((g.nbx + 3) / 4) * ((g.nby + 7) / 8) * nwin;  // of 4 x 8 blocks
     const bool fits[2] = {g.split[0].smem <= kMatchSmemMax, g.split[1].smem <= kMatchSmemMax};
     if (warps <= 160 && fits[1]) return 8;
-    if (warps <= (radius == 0 ? 600 : 450) && fits[0]) return 4;
+    const int few = radius == 0 ? (bm_range <= 2 ? 300 : 600) : 450;
+    if (warps <= few && fits[0]) return 4;
     return kSmemPerSm / (g.smem + 1024) * g.wx <= 4 && g.split[0].smem < g.smem / 2 ? 4 : 1;
 }
 
@@ -277,7 +284,7 @@ cudaError_t launch_match_split(const MatchParams &p, const MatchGeometry &g, int
 
 cudaError_t launch_match(const MatchParams &p, const MatchGeometry &g, int nwin,
                          cudaStream_t stream) {
-    const int lanes = match_lanes(g, p.radius, nwin);
+    const int lanes = match_lanes(g, p.bm_range, p.radius, nwin);
     if (p.metric != 0) {
         const int K = metric_strip_width(p.bm_range, p.radius, p.ps_num, p.ps_range);
         return launch_match_metric(p, g, nwin, K, lanes == 1 ? 1 : 4, stream);
