@@ -272,6 +272,7 @@ int prepare(bm3d_b200_batch *b) {
             f.radius = c.prm.radius;
             f.nblk = g.nbx * g.nby;
             f.nbx = g.nbx;
+            f.block_step = c.prm.block_step[0];
             f.nwin = N;
             f.corner_weight = 1;
             set_acc_pairs(f, c.d_acc, N, c.h);

@@ -190,6 +190,7 @@ int graph_enqueue(bm3d_b200_graph *g, cudaStream_t s, bool copies) {
         fp.radius = g->radius;
         fp.nblk = g->geo.nbx * g->geo.nby;
         fp.nbx = g->geo.nbx;
+        fp.block_step = g->block_step;
         fp.corner_weight = 0;
         set_acc_pairs(fp, g->d_res, g->nplanes * tw, g->height);
         fp.nwin = 1;
@@ -743,6 +744,7 @@ int clip_run_impl(bm3d_b200_clip *c, const float *d_src, const float *d_ref, flo
             fp.radius = r;
             fp.nblk = g.nbx * g.nby;
             fp.nbx = g.nbx;
+            fp.block_step = c->prm.block_step[pq];
             fp.corner_weight = raw ? 0 : 1;
             if (raw)
                 set_raw_pairs(fp, d_dst, N, c->raw_frame_floats, c->rawoff[q], Hq);
@@ -1022,6 +1024,7 @@ int run_stage_windows(bm3d_b200_clip *c, void **d_tab, float *d_mult, bool final
     fp.radius = r;
     fp.nblk = g.nbx * g.nby;
     fp.nbx = g.nbx;
+    fp.block_step = c->prm.block_step[0];
     fp.win0 = w0;
     fp.nwin = w1 - w0;
     fp.corner_weight = 1;
@@ -1672,6 +1675,7 @@ extern "C" int bm3d_b200_window_noalloc(float *d_res, const float *d_src, int wi
         fp.radius = radius;
         fp.nblk = (int)nblk;
         fp.nbx = geo.nbx;
+        fp.block_step = block_step;
         fp.corner_weight = 0;
         set_acc_pairs(fp, d_res, np * tw, height);
         fp.nwin = 1;
@@ -2113,6 +2117,7 @@ int stream_filter(bm3d_b200_stream *s, bm3d_b200_stream::Request &q,
             fp.radius = r;
             fp.nblk = s->geo[mq].nbx * s->geo[mq].nby;
             fp.nbx = s->geo[mq].nbx;
+            fp.block_step = s->prm.block_step[pq];
             fp.corner_weight = 0;
             set_raw_pairs(fp, s->d_raw, (long long)s->wslot.size(), s->raw_floats, s->rawoff[qq],
                           s->ph[qq]);

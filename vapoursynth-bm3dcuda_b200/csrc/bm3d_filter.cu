@@ -984,11 +984,22 @@ cudaError_t launch_filter_t(const FilterParams &p, const CUtensorMap &map, dim3 
     return cudaGetLastError();
 }
 
+// Where the eight block rows that cover a pixel are in flight at once, all of one
+// plane, the additions to the same words bound the kernel, and a weight box adds 96
+// words for a patch's 64 weights. (At block_step 1 up to 888 blocks a row, with 3
+// CTAs of 16 groups on each of 148 SMs. One window, hard threshold, us, as boxes / by
+// the load/store pipe: 413x186 288 / 265, 640x360 737 / 698, 850x200 509 / 508, 1000x250
+// 675 / 701. The Wiener kernel's own work hides the additions: 640x360 756 / 901.)
+bool crowded_windows(const FilterParams &p, bool final_) {
+    return !final_ && !p.corner_weight && p.radius == 0 && p.block_step == 1 &&
+           (long long)p.nwin * p.nbx * 8 <= 148 * 3 * kGroupsPerCta;
+}
+
 template <bool TC, bool VAR>
 cudaError_t launch_filter_form(const FilterParams &p, bool final_, dim3 grid,
                                cudaStream_t stream) {
     CUtensorMap map{};
-    if (!scatter_map(p, &map))
+    if ((!TC && crowded_windows(p, final_)) || !scatter_map(p, &map))
         return final_ ? launch_filter_t<true, TC, VAR, kScatterLsu>(p, map, grid, stream)
                       : launch_filter_t<false, TC, VAR, kScatterLsu>(p, map, grid, stream);
     if (p.corner_weight)

@@ -182,6 +182,7 @@ struct FilterParams {
     int nbx;  // blocks per block row (groups are scheduled row-major across windows)
     int win0;  // first window of this launch
     int nwin;  // windows win0 .. win0 + nwin - 1
+    int block_step;     // distance of the reference blocks
     int corner_weight;  // 1: add each patch's weight once at its top-left pixel
     float sigma;        // effective sigma (already scaled)
     float extractor;    // 2^extractor_exp, or 0
