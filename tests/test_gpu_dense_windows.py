@@ -1,6 +1,7 @@
-"""Windows of reference blocks at every pixel, on both sides of the line where the
-hard-threshold scatter leaves the boxes for the load/store pipe: the accumulators are
-the oracle's bit for bit (pre-rounded sums with room for 64 patches times 8)."""
+"""Windows on both sides of the lines where the hard-threshold scatter leaves the boxes
+for the load/store pipe (a block at every pixel; launches that save a wave by it): the
+accumulators are the oracle's bit for bit (pre-rounded sums with room for 64 patches
+times 8)."""
 import numpy as np
 import pytest
 
@@ -20,4 +21,16 @@ def test_accumulators(cuda, engine_lib, oracle, w, h, final, tx):
               transform_1d=tx)
     got = graph_run(win, ref, **kw)
     want = oracle.port_bm3d(win, ref, return_acc=True, **kw)
+    np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("w,h", [(227, 293), (245, 272), (227, 389), (242, 365)])
+def test_waves_of_other_transforms(cuda, engine_lib, oracle, w, h):
+    """444, 445, 592 and 593 CTAs; three planes."""
+    from bm3dcuda import synthetic as S
+    win = S.chroma_clip(1, h, w, seed=w)[0].transpose(1, 0, 2, 3).copy()
+    kw = dict(sigma=[7.0, 4.0, 4.0], radius=0, block_step=3, bm_range=2, extractor_exp=8,
+              chroma=True, transform_2d=2, transform_1d=1)
+    got = graph_run(win, **kw)
+    want = oracle.port_bm3d(win, return_acc=True, **kw)
     np.testing.assert_array_equal(got, want)

@@ -995,11 +995,25 @@ bool crowded_windows(const FilterParams &p, bool final_) {
            (long long)p.nwin * p.nbx * 8 <= 148 * 3 * kGroupsPerCta;
 }
 
+// The weight boxes leave room for 3 CTAs on an SM. Hard thresholding with the other
+// transforms runs 4 by the load/store pipe and is little slower by that: it takes that
+// form in small launches where the fourth place saves a wave. (One window, Hadamard,
+// radius 0, us, as boxes / by the load/store pipe: 357 CTAs 39.0 / 37.0, 510 51.6 / 41.3, 586
+// 59.0 / 48.1, 770 61.7 / 69.6, 1094 81.0 / 76.2, 1598 103.6 / 101.3, 3600 195.8 / 197.2. The
+// DCT's form of 5 gains less by its places: 586 44.6 / 41.6, 1094 59.9 / 65.8.)
+template <bool VAR>
+bool weight_boxes_cost_a_wave(const FilterParams &p, bool final_, long long ctas) {
+    const int boxes = 148 * 3, lsu = 148 * 4;
+    return VAR && !final_ && !p.corner_weight && ctas <= 2 * lsu &&
+           (ctas + boxes - 1) / boxes > (ctas + lsu - 1) / lsu;
+}
+
 template <bool TC, bool VAR>
 cudaError_t launch_filter_form(const FilterParams &p, bool final_, dim3 grid,
                                cudaStream_t stream) {
     CUtensorMap map{};
-    if ((!TC && crowded_windows(p, final_)) || !scatter_map(p, &map))
+    if ((!TC && crowded_windows(p, final_)) ||
+        weight_boxes_cost_a_wave<VAR>(p, final_, grid.x) || !scatter_map(p, &map))
         return final_ ? launch_filter_t<true, TC, VAR, kScatterLsu>(p, map, grid, stream)
                       : launch_filter_t<false, TC, VAR, kScatterLsu>(p, map, grid, stream);
     if (p.corner_weight)
