@@ -99,7 +99,7 @@ __device__ __forceinline__ void umma_k64(uint32_t d, uint32_t a_s, uint32_t b_s)
 }
 
 template <bool FINAL>
-__global__ void __launch_bounds__(kTThreads, FINAL ? 3 : 4) filter_tc_kernel(FilterParams prm) {
+__global__ void __launch_bounds__(kTThreads, FINAL ? 3 : 4) filter_tc_kernel(FilterCore prm) {
     extern __shared__ __align__(1024) unsigned char tsm[];
     constexpr uint32_t kRegion = tc_region<FINAL>();
     unsigned char *a0 = tsm;                              // noisy patches, then inverse operand
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(kTThreads, FINAL ? 3 : 4) filter_tc_kernel(Fil
 }
 
 template <bool FINAL>
-cudaError_t launch_tc(const FilterParams &p, unsigned grid, cudaStream_t stream) {
+cudaError_t launch_tc(const FilterCore &p, unsigned grid, cudaStream_t stream) {
     static int configured[64] = {};
     cudaError_t e = raise_smem_limit(configured, (const void *)filter_tc_kernel<FINAL>,
                                      tc_smem<FINAL>());
