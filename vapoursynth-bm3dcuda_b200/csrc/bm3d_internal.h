@@ -167,11 +167,11 @@ struct MatchBatch {
 cudaError_t launch_match_batch(const MatchBatch &b, int K, int kt, bool small, int wx, size_t smem,
                                cudaStream_t stream);
 
-// Collaborative filtering + scatter of one plane over a batch of windows: what every
-// form of the kernel reads. At most 128 bytes: by-value parameters above that are not
-// split into scalars, and the tensor-core kernel, which takes this part alone, ran
-// 2 to 5% slower for it (8 windows of 1920x1080, radius 2: 1018 us Wiener, 1074).
-struct FilterCore {
+// Collaborative filtering + scatter of one plane over a batch of windows. At most 128
+// bytes: a by-value kernel parameter above that is not split into scalars (at 136: 1080p
+// windows of radius 0, Hadamard, hard threshold 96.9 us instead of 93.5, Wiener 127.8
+// instead of 123.6).
+struct FilterParams {
     const float *const *src;  // [nwin][2r+1] noisy planes of the filtered plane
     const float *const *ref;  // [nwin][2r+1] basic-estimate planes (final stage) or null
     float *const *acc;        // [nwin][2r+1] wdst plane receiving slot z, or null (dropped)
@@ -185,25 +185,22 @@ struct FilterCore {
     int nbx;  // blocks per block row (groups are scheduled row-major across windows)
     int win0;  // first window of this launch
     int nwin;  // windows win0 .. win0 + nwin - 1
-    int corner_weight;  // 1: add each patch's weight once at its top-left pixel
     float sigma;        // effective sigma (already scaled)
     float extractor;    // 2^extractor_exp, or 0
-    int precision;      // 0: FP32, the reference's factorisation; 1: split-BF16 tensor
-                        // cores; 2: FP16 Kronecker-form 2-D transforms on tcgen05
-    int t2d, t1d;       // transforms (rows/columns, group): 0 DCT, 1 Haar, 2 WHT, 3 bior1.5
-    unsigned *err;      // precision 2: set to nonzero when a CTA gave up waiting for its MMAs
-};
-static_assert(sizeof(FilterCore) <= 128, "split into scalars as a kernel parameter");
-
-struct FilterParams : FilterCore {
+    signed char corner_weight;  // 1: add each patch's weight once at its top-left pixel
+    signed char precision;  // 0: FP32, the reference's factorisation; 1: split-BF16 tensor
+                            // cores; 2: FP16 Kronecker-form 2-D transforms on tcgen05
+    signed char t2d, t1d;  // transforms (rows/columns, group): 0 DCT, 1 Haar, 2 WHT, 3 bior1.5
     // The targets of `acc` when they all lie in one allocation as acc_pairs pairs
     // of a wdst and a weight plane (acc_pair_rows rows of acc_stride floats
     // together), or a null acc_base: what the scatter by TMA needs.
     float *acc_base;
     int acc_pairs, acc_pair_rows;
     float acc_pair_inv;  // 1 / (acc_pair_rows * acc_stride)
-    int block_step;      // distance of the reference blocks
+    int block_step;     // distance of the reference blocks
+    unsigned *err;      // precision 2: set to nonzero when a CTA gave up waiting for its MMAs
 };
+static_assert(sizeof(FilterParams) <= 128, "split into scalars as a kernel parameter");
 
 // Sets the fields that describe the accumulator pairs (rows: of one plane).
 inline void set_acc_pairs(FilterParams &p, float *base, int pairs, int rows) {
