@@ -668,7 +668,7 @@ def run_our_arm(args, rank: int, world: int, dist):
             peaks["source"], "196,608 tensor FLOP per group (two forward 2-D transforms and "
             "the inverse)", bound="tensor")
     else:
-        fb, ff_ = "filter_kernel<0,0,0>", "filter_kernel<1,0,0>"
+        fb, ff_ = "filter_kernel<0,0,0,1>", "filter_kernel<1,0,0,1>"
         kernels[fb] = entry(
             fb, groups * 18240, "TFLOP/s", per_launch(head, 1), peak, fp32_src,
             "18,240 FLOP per group (3-D DCT forward + inverse, FFTW operation counts x 192 "
@@ -680,8 +680,8 @@ def run_our_arm(args, rank: int, world: int, dist):
         "aggregate_kernel", 12 * W * H * frames, "GB/s", per_launch(head, 2),
         peaks["hbm_gbs"], peaks["source"],
         "12 B per pixel (weighted sum and corner weights read, output written)", bound="hbm")
-    kernels["match_kernel<10,0>"] = entry(
-        "match_kernel<10,0>", SSD_FLOP * cand * frames, "TFLOP/s", per_launch(plain, 0), peak,
+    kernels["match_kernel<10,9,0,1,1,3>"] = entry(
+        "match_kernel<10,9,0,1,1,3>", SSD_FLOP * cand * frames, "TFLOP/s", per_launch(plain, 0), peak,
         fp32_src, "exhaustive search (plain arm): 192 FLOP per candidate")
     kernels = {k: v for k, v in kernels.items() if v is not None}
     # the headline roofline: the kernel with the largest share of the headline step
@@ -692,7 +692,7 @@ def run_our_arm(args, rank: int, world: int, dist):
         if k in kernels:
             share[k] = float(head["stage_ms"][i])
     if prop is None:
-        share["match_kernel<10,0>"] = float(head["stage_ms"][0])
+        share["match_kernel<10,9,0,1,1,3>"] = float(head["stage_ms"][0])
     top = max(share, key=share.get)
     roofline = dict(kernels[top])
     roofline["share_of_step"] = share[top] / sum(head["stage_ms"])

@@ -17,14 +17,19 @@
 // column frequency, in-register index = group frequency * 8 + row frequency),
 // so the Wiener weight's sum of squares is accumulated in the same order.
 //
-// Scatter: where the accumulators lie in one allocation with corner weights
-// (the clip and batch paths; scatter_map has the conditions), each patch goes as
-// one TMA reduction of a 12 x 8 box, which takes the 64 additions per thread off
-// the load/store pipe. Elsewhere (raw stacks, single windows) the 8 threads of a
-// group add 8 contiguous pixels of a patch row per instruction. With
-// corner weights the weight of a patch is added once, at its top-left pixel;
-// the aggregation kernel then sums each pixel's 8x8 neighbourhood of corners,
-// which equals the per-pixel weight sum (exactly so with pre-rounding).
+// Scatter, in three forms (launch_filter_form chooses):
+//   boxes with corner weights (clips and batches): each patch goes as one TMA
+//     reduction of a 12 x 8 box, which takes the 64 additions per thread off the
+//     load/store pipe; the weight of a patch is added once, at its top-left pixel,
+//     and the aggregation kernel sums each pixel's 8x8 neighbourhood of corners,
+//     which equals the per-pixel weight sum (exactly so with pre-rounding);
+//   boxes with a weight for every pixel (single windows, raw stacks, streams): a
+//     second box per patch;
+//   the load/store pipe: the 8 threads of a group add 8 contiguous pixels of a
+//     patch row per instruction. For layouts that boxes cannot address (scatter_map:
+//     row strides that are no multiple of 4, bases off a 16-byte boundary, raw planes
+//     that do not line up, 2^20 accumulators and more) and for the hard-threshold
+//     windows where it is faster (crowded_windows, weight_boxes_cost_a_wave).
 //
 // Groups are scheduled block-row-major across windows: CTAs running together
 // work on the same rows of every window, so the gathered patches and the
@@ -33,11 +38,10 @@
 // Bound: the load/store pipe and the issue slots, then the L2's additions. Of
 // the 30-window 1920x1080 radius-2 launches (hard threshold / Wiener): gathers
 // alone take 0.30 / 0.60 ms, the additions alone 0.57 (as reductions of the
-// load/store pipe) or 0.70 (TMA, in parallel). 1.25 / 2.41 ms before, 1.09 /
-// 1.98 with the scatter by TMA, 0.97 / 1.79 with the paired layout exchanges,
-// 0.99 / 1.73 with packed scatter arithmetic kept exact and the prefetch loop
-// rolled: at 48 KB of code the Wiener kernel's warps waited for instructions
-// (1.4 stalls per issue, 0.44 after).
+// load/store pipe) or 0.70 (TMA, in parallel). The launches take 0.99 / 1.73 ms
+// (1.25 / 2.41 with the load/store scatter, single-word exchanges and an unrolled
+// prefetch, by which the Wiener kernel had 48 KB of code and its warps waited 1.4
+// cycles an issue for instructions, 0.44 now).
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -406,11 +410,10 @@ __device__ __forceinline__ void scatter_lsu(const FilterParams &prm, const float
                                             const int (&pos)[8], int win, bool active, int me,
                                             int g) {
     const int tw = 2 * prm.radius + 1;
-    // thread `me` owns column
-    // `me` of every patch and adds one patch per iteration of a rolled loop
-    // (the patch position comes from lane `p` of the group). Pre-rounding with
-    // 2^extractor_exp makes the sums independent of the atomic order; a
-    // multiplicity of 1 multiplies exactly.
+    // Thread `me` owns column `me` of every patch and adds one patch per
+    // iteration of a rolled loop (the patch position comes from lane `p` of the
+    // group). Pre-rounding with 2^extractor_exp makes the sums independent of the
+    // atomic order; a multiplicity of 1 multiplies exactly.
     // Lane `me` resolves patch `me`'s target (plane pointer, multiplicity)
     // once; the loop takes patch p's from lane p of the group.
     const int pos_me = pick_pos(pos, me);
@@ -463,14 +466,7 @@ __device__ __forceinline__ void store_box_row(float *row, const float (&v)[8], i
             make_float4(u[4 * i], u[4 * i + 1], u[4 * i + 2], u[4 * i + 3]);
 }
 
-// Weighted scatter of a warp's four groups by TMA reductions (thread = row `me`
-// of group g, v[p][column]): each patch goes as one 8 x 12 box added to the
-// accumulators, from the 16-byte boundary at or below its first pixel, so
-// that the additions leave the load/store pipe, which bounds the filter. Lane
-// `me` issues patch `me`'s box. Same terms as scatter_lsu.
-// WEIGHTS: the patch's weight goes to all its pixels, as a second box from the
-// one of four (one per column offset) that the group fills with its weight;
-// multiplicities are 1. Else once, at the patch's corner.
+// Adds a 12 x 8 box of shared memory to the accumulators at (x, y) of the map.
 __device__ __forceinline__ void reduce_box(const CUtensorMap *map, int x, int y, const float *box) {
     asm volatile(
         "cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], "
@@ -479,6 +475,14 @@ __device__ __forceinline__ void reduce_box(const CUtensorMap *map, int x, int y,
         : "memory");
 }
 
+// Weighted scatter of a warp's four groups by TMA reductions (thread = row `me`
+// of group g, v[p][column]): each patch goes as one 8 x 12 box added to the
+// accumulators, from the 16-byte boundary at or below its first pixel, so
+// that the additions leave the load/store pipe, which bounds the filter. Lane
+// `me` issues patch `me`'s box. Same terms as scatter_lsu.
+// WEIGHTS: the patch's weight goes to all its pixels, as a second box from the
+// one of four (one per column offset) that the group fills with its weight;
+// multiplicities are 1. Else once, at the patch's corner.
 template <bool WEIGHTS>
 __device__ __forceinline__ void scatter_tma(const FilterParams &prm, const CUtensorMap *map,
                                             float *box, const float (&v)[8][8], float weight,
@@ -706,11 +710,10 @@ __device__ __forceinline__ void filter_cta(const FilterParams &prm, const CUtens
         scatter_lsu<TC>(prm, S, weight, pos, win, active, me, g);
 }
 
-
-// Resident CTAs per SM the register allocation aims at: the hard-threshold
-// FP32 kernel fits 96 registers without spills (5 CTAs: 1.30 ms against 1.33
-// at 4 for the 30-window launch), its TMA form's boxes allow 4; the Wiener
-// kernel's shared memory allows 3.
+// Resident CTAs per SM the register allocation aims at: the load/store form of the
+// hard-threshold FP32 kernel runs 5 at 96 registers, 12 bytes of them spilled (one
+// 640x360 window, block_step 1: 638 us, 675 at 4 without spills); boxes leave room
+// for 4, with weights 3; the Wiener kernel's shared memory allows 3.
 template <bool FINAL, bool TC, bool VAR, int SC>
 constexpr int filter_ctas_per_sm() {
     return FINAL || SC == kScatterWeights ? 3 : (TC || VAR || SC == kScatterBoxes ? 4 : 5);
@@ -759,8 +762,8 @@ __global__ void __launch_bounds__(128, filter_ctas_per_sm<FINAL, false, false, k
 }
 
 // dst = wdst / weight; with corner weights the weight of a pixel is the sum of
-// the corner plane over its 8x8 up-left neighbourhood. A CTA handles a 32x8
-// output tile; corner sums run vertically then horizontally in a fixed order.
+// the corner plane over its 8x8 up-left neighbourhood; corner sums run
+// vertically then horizontally in a fixed order.
 // A CTA of 256 threads covers a 128 x 16 tile; each thread 8 consecutive
 // pixels of one row, loaded and stored as float4 pairs when aligned.
 constexpr int kAggTx = 128, kAggTy = 16, kAggThreads = 256;

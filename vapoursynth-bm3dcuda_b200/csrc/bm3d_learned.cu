@@ -158,8 +158,8 @@ __device__ __forceinline__ void rank_cells(unsigned (&keys)[K], const uint4 er,
 
 // SMALL (ps_num <= 2, or no neighbour frames): a neighbour frame's list keeps
 // two entries, all that is ever read of it, and the block's list lies in shared
-// memory while a stage ranks and scores (168 registers: 412 bytes spilled
-// before, 132 now).
+// memory while a stage ranks and scores (at 168 registers 144 to 176 bytes are
+// spilled, 408 to 452 without).
 template <int K, bool SMALL>
 __device__ void learned_tile(const MatchParams &p, const LearnedParams &lp, int tile_x,
                              int tile_y, int win, float *tile) {
@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(128, 3) learned_match_kernel(MatchParams p, Le
     const unsigned id = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
     const unsigned rest = id / gridDim.x;
     learned_tile<K, SMALL>(p, lp, (int)(id % gridDim.x), (int)(rest / gridDim.z),
-                    p.win0 + (int)(rest % gridDim.z), tile);
+                           p.win0 + (int)(rest % gridDim.z), tile);
 }
 
 // ---------------------------------------------------------------------------
