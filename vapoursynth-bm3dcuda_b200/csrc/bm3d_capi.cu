@@ -1280,8 +1280,7 @@ extern "C" int bm3d_b200_clip_set_proposer(bm3d_b200_clip *c, bm3d_b200_proposer
     const int N = c->nframes, r = c->prm.radius, tw = 2 * r + 1;
     const size_t ntab = (size_t)N * tw;
     const MatchGeometry lg = learned_geometry(c->pw[0], c->ph[0], c->prm.block_step[0],
-                                              c->prm.bm_range[0], r, c->prm.ps_num[0],
-                                              c->prm.ps_range[0]);
+                                              c->prm.bm_range[0], r, c->prm.ps_range[0]);
     if (lg.smem > kMatchSmemMax ||
         !learned_ordinals_fit(c->prm.bm_range[0], c->prm.ps_num[0], c->prm.ps_range[0]))
         return fail(BM3D_B200_ERR_UNSUPPORTED, "BM3D: search range too large for learned matching");
@@ -1437,7 +1436,7 @@ extern "C" int bm3d_b200_learned_match(const float *const *d_frames, const void 
         return fail(BM3D_B200_ERR_INVALID, "BM3D: proposal cell counts must be in range [1, 8]");
     const int tw = 2 * radius + 1;
     const MatchGeometry g = match_geometry(width, height, block_step, bm_range, radius, ps_num, ps_range);
-    const MatchGeometry lg = learned_geometry(width, height, block_step, bm_range, radius, ps_num,
+    const MatchGeometry lg = learned_geometry(width, height, block_step, bm_range, radius,
                                               ps_range);
     if (lg.smem > kMatchSmemMax || !learned_ordinals_fit(bm_range, ps_num, ps_range))
         return fail(BM3D_B200_ERR_UNSUPPORTED, "BM3D: search range too large for learned matching");
@@ -2618,8 +2617,7 @@ extern "C" int bm3d_b200_stream_set_proposer(bm3d_b200_stream *s, bm3d_b200_prop
     stream_wait_idle(s, lk);
     if (p) {
         const MatchGeometry lg = learned_geometry(s->pw[0], s->ph[0], s->prm.block_step[0],
-                                                  s->prm.bm_range[0], s->r, s->prm.ps_num[0],
-                                                  s->prm.ps_range[0]);
+                                                  s->prm.bm_range[0], s->r, s->prm.ps_range[0]);
         if (lg.smem > kMatchSmemMax ||
             !learned_ordinals_fit(s->prm.bm_range[0], s->prm.ps_num[0], s->prm.ps_range[0]))
             return fail(BM3D_B200_ERR_UNSUPPORTED,

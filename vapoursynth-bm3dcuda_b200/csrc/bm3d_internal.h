@@ -132,7 +132,7 @@ struct LearnedParams {
     unsigned fallback_capacity;
 };
 MatchGeometry learned_geometry(int width, int height, int block_step, int bm_range, int radius,
-                               int ps_num, int ps_range);
+                               int ps_range);
 cudaError_t launch_learned_match(const MatchParams &p, const LearnedParams &lp,
                                  const MatchGeometry &g, int nwin, cudaStream_t stream);
 // Whether every candidate cell of a stage gets a distinct 12-bit ordinal

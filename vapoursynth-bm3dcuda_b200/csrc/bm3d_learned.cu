@@ -109,14 +109,12 @@ __device__ __forceinline__ CellRect cell_rect(const Box &b) {
 // Ranks the cells of search window i of a stage into `keys`, skipping cells
 // that an earlier window's cell rectangle already held (b0: window 0's box;
 // windows 1 .. i-1 are recomputed from their centres in `last`). ord0: the
-// ordinal of the window's first cell. The cells are walked in order, kRankBatch
-// at a time with their loads issued first (30 windows of 1920x1080, radius 2:
-// 1.96 ms; 1.99 with four loads in flight and single ones for a row's remainder);
-// a skipped cell inserts the empty key (a no-op of the min/max network),
-// so the walk has no divergent branch.
-constexpr int kRankBatch = 8;
-
-template <int K, int N>
+// ordinal of the window's first cell. A skipped cell inserts the empty key (a
+// no-op of the min/max network), so the walk has no divergent branch. The
+// window's cell rows are walked one by one, four cells per iteration with their
+// loads issued first and a row's remainder one by one; FLAT: eight cells per
+// iteration across row ends (flat_ranking says where).
+template <bool FLAT, int K, int N>
 __device__ __forceinline__ void rank_cells(unsigned (&keys)[K], const uint4 er,
                                            const uint4 *__restrict__ emb, int w2, const Box &bi,
                                            unsigned ord0, int i, const Box &b0,
@@ -131,27 +129,51 @@ __device__ __forceinline__ void rank_cells(unsigned (&keys)[K], const uint4 er,
             seen |= in_cells(stage_box(p, st, x, y, m, range, pick(last, j)), gx, gy);
         return seen;
     };
-    const int ncol = cr.gx1 - cr.gx0 + 1, n = ncol * (cr.gy1 - cr.gy0 + 1);
-    int gx = cr.gx0, gy = cr.gy0;
-    const uint4 *cell = cell_ptr(emb, w2, gx, gy);
-    for (int c = 0; c < n; c += kRankBatch) {
-        uint4 e[kRankBatch];
-        bool skip[kRankBatch];
+    const int ncol = cr.gx1 - cr.gx0 + 1;
+    if constexpr (FLAT) {
+        constexpr int kBatch = 8;
+        const int n = ncol * (cr.gy1 - cr.gy0 + 1);
+        int gx = cr.gx0, gy = cr.gy0;
+        const uint4 *cell = cell_ptr(emb, w2, gx, gy);
+        for (int c = 0; c < n; c += kBatch) {
+            uint4 e[kBatch];
+            bool skip[kBatch];
 #pragma unroll
-        for (int j = 0; j < kRankBatch; ++j) {
-            e[j] = __ldg(cell);
-            skip[j] = c + j >= n || seen_earlier(gx, gy);
-            if (c + j + 1 < n) {  // the last cell is loaded again past the end
-                const bool wrap = gx == cr.gx1;
-                gx = wrap ? cr.gx0 : gx + 1;
-                gy += wrap;
-                cell += wrap ? w2 - ncol + 1 : 1;
+            for (int j = 0; j < kBatch; ++j) {
+                e[j] = __ldg(cell);
+                skip[j] = c + j >= n || seen_earlier(gx, gy);
+                if (c + j + 1 < n) {  // the last cell is loaded again past the end
+                    const bool wrap = gx == cr.gx1;
+                    gx = wrap ? cr.gx0 : gx + 1;
+                    gy += wrap;
+                    cell += wrap ? w2 - ncol + 1 : 1;
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < kBatch; ++j) {
+                const unsigned key = (emb_dist(er, e[j]) << kOrdinalBits) | (ord0 + c + j);
+                key_insert(keys, skip[j] ? kNoKey : key);
             }
         }
+        return;
+    }
+    unsigned o = ord0;
+    for (int gy = cr.gy0; gy <= cr.gy1; ++gy, o += (unsigned)ncol) {
+        const uint4 *row = cell_ptr(emb, w2, cr.gx0, gy);
+        int k = 0;
+        for (; k + 3 < ncol; k += 4) {
+            uint4 e[4];
 #pragma unroll
-        for (int j = 0; j < kRankBatch; ++j) {
-            const unsigned key = (emb_dist(er, e[j]) << kOrdinalBits) | (ord0 + c + j);
-            key_insert(keys, skip[j] ? kNoKey : key);
+            for (int j = 0; j < 4; ++j) e[j] = __ldg(row + k + j);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const unsigned key = (emb_dist(er, e[j]) << kOrdinalBits) | (o + k + j);
+                key_insert(keys, seen_earlier(cr.gx0 + k + j, gy) ? kNoKey : key);
+            }
+        }
+        for (; k < ncol; ++k) {
+            const unsigned key = (emb_dist(er, __ldg(row + k)) << kOrdinalBits) | (o + k);
+            key_insert(keys, seen_earlier(cr.gx0 + k, gy) ? kNoKey : key);
         }
     }
 }
@@ -160,7 +182,7 @@ __device__ __forceinline__ void rank_cells(unsigned (&keys)[K], const uint4 er,
 // two entries, all that is ever read of it, and the block's list lies in shared
 // memory while a stage ranks and scores (at 168 registers 144 to 176 bytes are
 // spilled, 408 to 452 without).
-template <int K, bool SMALL>
+template <int K, bool SMALL, bool FLAT>
 __device__ void learned_tile(const MatchParams &p, const LearnedParams &lp, int tile_x,
                              int tile_y, int win, float *tile) {
     const int lane = threadIdx.x & 31;
@@ -239,7 +261,7 @@ __device__ void learned_tile(const MatchParams &p, const LearnedParams &lp, int 
             unsigned ord0 = 0;
             for (int i = 0; i < nwin; ++i) {
                 const Box bi = i == 0 ? b0 : stage_box(p, st, x, y, m, range, pick(last, i));
-                rank_cells(keys, er, emb, lp.w2, bi, ord0, i, b0, p, st, x, y, m, range, last);
+                rank_cells<FLAT>(keys, er, emb, lp.w2, bi, ord0, i, b0, p, st, x, y, m, range, last);
                 const CellRect cr = cell_rect(bi);
                 ord0 += (unsigned)((cr.gx1 - cr.gx0 + 1) * (cr.gy1 - cr.gy0 + 1));
             }
@@ -347,12 +369,12 @@ __device__ void learned_tile(const MatchParams &p, const LearnedParams &lp, int 
 // band of tile rows in every window before the next band, so the CTAs that
 // run together read the same rows of the (shared) frames and embeddings and
 // those stay in L2 (window-major order re-reads them from DRAM).
-template <int K, bool SMALL>
+template <int K, bool SMALL, bool FLAT>
 __global__ void __launch_bounds__(128, 3) learned_match_kernel(MatchParams p, LearnedParams lp) {
     extern __shared__ float tile[];
     const unsigned id = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
     const unsigned rest = id / gridDim.x;
-    learned_tile<K, SMALL>(p, lp, (int)(id % gridDim.x), (int)(rest / gridDim.z),
+    learned_tile<K, SMALL, FLAT>(p, lp, (int)(id % gridDim.x), (int)(rest / gridDim.z),
                            p.win0 + (int)(rest % gridDim.z), tile);
 }
 
@@ -614,29 +636,28 @@ cudaError_t launch_rescore(const MatchParams &p, int nwin, cudaStream_t stream) 
 }
 
 MatchGeometry learned_geometry(int width, int height, int block_step, int bm_range, int radius,
-                               int ps_num, int ps_range) {
+                               int ps_range) {
     MatchGeometry g{};
     g.nbx = (width - 8 + block_step - 1) / block_step + 1;
     g.nby = (height - 8 + block_step - 1) / block_step + 1;
     const int mmax = bm_range + radius * ps_range;
     g.tile_rows = 7 * block_step + 2 * mmax + 10;
     g.ks = g.kt = 2;
-    g.small = radius == 0 || ps_num <= 2;
-    auto bytes = [&](int pitch, int wx, int words) {
-        return (size_t)pitch * g.tile_rows * sizeof(float) + (size_t)words * 32 * wx * sizeof(int);
+    auto bytes = [&](int pitch, int wx) {
+        return (size_t)pitch * g.tile_rows * sizeof(float) + (size_t)8 * 32 * wx * sizeof(int);
     };
-    // a range whose one-warp CTA needs more than 220 KB (with 8 list words per
-    // thread) is refused
-    if (bytes(3 * block_step + 2 * mmax + 18, 1, 8) > kMatchSmemLimit) {
+    // a range whose one-warp CTA needs more than 220 KB is refused
+    if (bytes(3 * block_step + 2 * mmax + 18, 1) > kMatchSmemLimit) {
         g.wx = 1;
         g.smem = kMatchSmemMax + 1;
         return g;
     }
-    // the CTA width with the most resident warps, the widest of equals
+    // the CTA width with the most resident warps, the widest of equals (6 windows of
+    // 1920x1080, radius 2, bm_range 16: 851 us; 1213 with the widest of up to 72 KB)
     int best = 0;
     for (int wx = 4; wx >= 1; wx /= 2) {
         const int pitch = (4 * wx - 1) * block_step + 2 * mmax + 17;
-        const size_t smem = bytes(pitch, wx, g.small ? 16 : 8);
+        const size_t smem = bytes(pitch, wx);
         const int warps = std::min<int>(12, (int)(228 * 1024 / (smem + 1024)) * wx);
         if (warps > best && smem <= kMatchSmemMax) {
             best = warps;
@@ -655,35 +676,63 @@ bool learned_ordinals_fit(int bm_range, int ps_num, int ps_range) {
     return sp <= (1 << kOrdinalBits) && tp <= (1 << kOrdinalBits);
 }
 
-template <int K, bool SMALL>
+namespace {
+
+template <int K, bool SMALL, bool FLAT>
 cudaError_t launch_learned_k(const MatchParams &p, const LearnedParams &lp, const MatchGeometry &g,
-                             int nwin, cudaStream_t stream) {
+                             size_t smem, int nwin, cudaStream_t stream) {
     static int configured[64] = {0};
-    cudaError_t e =
-        raise_smem_limit(configured, (const void *)learned_match_kernel<K, SMALL>, g.smem);
+    const auto fn = learned_match_kernel<K, SMALL, FLAT>;
+    cudaError_t e = raise_smem_limit(configured, (const void *)fn, smem);
     if (e != cudaSuccess) return e;
     dim3 block(32 * g.wx);
     dim3 grid((p.nbx + 4 * g.wx - 1) / (4 * g.wx), (p.nby + 7) / 8, nwin);
-    learned_match_kernel<K, SMALL><<<grid, block, g.smem, stream>>>(p, lp);
+    fn<<<grid, block, smem, stream>>>(p, lp);
     return cudaGetLastError();
 }
 
-template <bool SMALL>
+template <bool SMALL, bool FLAT>
 cudaError_t launch_learned_s(const MatchParams &p, const LearnedParams &lp, const MatchGeometry &g,
-                             int nwin, cudaStream_t stream) {
+                             size_t smem, int nwin, cudaStream_t stream) {
     const int cells = std::max(lp.cells_s, lp.cells_t);
-    if (cells <= 2) return launch_learned_k<2, SMALL>(p, lp, g, nwin, stream);
-    return cells <= 4 ? launch_learned_k<4, SMALL>(p, lp, g, nwin, stream)
-                      : launch_learned_k<8, SMALL>(p, lp, g, nwin, stream);
+    if (cells <= 2) return launch_learned_k<2, SMALL, FLAT>(p, lp, g, smem, nwin, stream);
+    return cells <= 4 ? launch_learned_k<4, SMALL, FLAT>(p, lp, g, smem, nwin, stream)
+                      : launch_learned_k<8, SMALL, FLAT>(p, lp, g, smem, nwin, stream);
 }
+
+// Whether cells are ranked across row ends: where fours leave a fifth of a temporal
+// window's row or more to single loads, in windows wider than four cells, and the
+// lanes' windows lie more than two cells apart (two-stage clips on moving texture, all
+// stages, across row ends / row by row, us: block_step 8: ps_range 3 1173 / 1117, 4 6223
+// / 6259, 5 1136 / 1172, 6 1206 / 1259, 8 824 / 816; block_step 4: ps_range 4 1446 / 1430;
+// block_step 1, the search alone, 644x228: ps_range 6 287 / 260).
+bool flat_ranking(int ps_range, int block_step) {
+    const int columns = ps_range + 1;
+    return block_step > 4 && columns > 4 && 5 * (columns % 4) >= columns;
+}
+
+}  // namespace
 
 cudaError_t launch_learned_match(const MatchParams &p, const LearnedParams &lp,
                                  const MatchGeometry &g, int nwin, cudaStream_t stream) {
     if (g.smem > kMatchSmemMax || lp.cells_s < 1 || lp.cells_s > 8 || lp.cells_t < 1 ||
         lp.cells_t > 8 || !learned_ordinals_fit(p.bm_range, p.ps_num, p.ps_range))
         return cudaErrorInvalidValue;
-    return g.small ? launch_learned_s<true>(p, lp, g, nwin, stream)
-                   : launch_learned_s<false>(p, lp, g, nwin, stream);
+    // The short lists where they apply, cost no resident CTA and the launch has warps
+    // (of 4 x 8 blocks) for the registers they save: over random searches with ps_num
+    // <= 2 they take 0.97 of the general form's time from 1000 warps on, 1.01 below
+    // (1.08 at worst), 1.01 at radius 0.
+    const size_t small_smem = g.smem + (size_t)8 * 32 * g.wx * sizeof(int);
+    const auto resident = [&](size_t smem) {
+        return std::min<int>(12 / g.wx, (int)(228 * 1024 / (smem + 1024)));
+    };
+    const long long warps = (long long)((p.nbx + 3) / 4) * ((p.nby + 7) / 8) * nwin;
+    if (p.radius > 0 && p.ps_num <= 2 && warps >= 1000 && small_smem <= kMatchSmemMax &&
+        resident(small_smem) == resident(g.smem))
+        return flat_ranking(p.ps_range, p.block_step)
+                   ? launch_learned_s<true, true>(p, lp, g, small_smem, nwin, stream)
+                   : launch_learned_s<true, false>(p, lp, g, small_smem, nwin, stream);
+    return launch_learned_s<false, false>(p, lp, g, g.smem, nwin, stream);
 }
 
 cudaError_t launch_match_fallback(const MatchParams &p, const unsigned *list,
