@@ -173,7 +173,7 @@ def test_batch_of_more_frames_than_boxes_count(cuda, engine_lib):
     (16, 0, 16), (13, 0, 16), (15, 0, 16), (16, 1, 16), (16, 0, 17)])
 @pytest.mark.parametrize("radius", [1, 3])
 def test_vaggregate_layouts(cuda, engine_lib, radius, raw_stride, offset, dst_stride):
-    """Quads of pixels (the first layout) and single pixels."""
+    """Single pixels (narrow rows), at every stride and offset."""
     import torch
     from bm3dcuda import _lib
     h, w, tw = 11, 13, 2 * radius + 1
@@ -197,5 +197,35 @@ def test_vaggregate_layouts(cuda, engine_lib, radius, raw_stride, offset, dst_st
     for i in range(tw):
         sv += raws[i, tw - 1 - i, 0]
         sw += raws[i, tw - 1 - i, 1]
+    np.testing.assert_array_equal(got[:, :w], sv / sw)
+    assert (got[:, w:] == 5.0).all()
+
+
+@pytest.mark.parametrize("w,stride,offset", [(128, 128, 0), (129, 132, 0), (131, 132, 0),
+                                             (132, 132, 0), (515, 516, 0), (640, 640, 0),
+                                             (640, 640, 1), (639, 639, 0)])
+@pytest.mark.parametrize("radius", [0, 2, 3])
+def test_vaggregate_widths(cuda, engine_lib, radius, w, stride, offset):
+    """Rows of one block and more: quads from 129 columns on, with every remainder."""
+    import torch
+    from bm3dcuda import _lib
+    h, tw = 5, 2 * radius + 1
+    rng = np.random.default_rng(w)
+    raws = rng.uniform(0.5, 2.0, (tw, tw, 2, h, stride)).astype(np.float32)
+    keep, ptrs = [], (ctypes.c_void_p * tw)()
+    for i in range(tw):
+        buf = torch.zeros(raws[i].size + offset, device="cuda")
+        buf[offset:] = torch.from_numpy(raws[i].reshape(-1)).cuda()
+        keep.append(buf)
+        ptrs[i] = buf.data_ptr() + 4 * offset
+    dst = torch.full((h, stride), 5.0, device="cuda")
+    _lib.check(engine_lib.bm3d_b200_vaggregate(dst.data_ptr(), stride, ptrs, stride, w, h, radius,
+                                               radius, tw, None))
+    torch.cuda.synchronize()
+    got = dst.cpu().numpy()
+    sv, sw = np.zeros((h, w), np.float32), np.zeros((h, w), np.float32)
+    for i in range(tw):
+        sv += raws[i, tw - 1 - i, 0, :, :w]
+        sw += raws[i, tw - 1 - i, 1, :, :w]
     np.testing.assert_array_equal(got[:, :w], sv / sw)
     assert (got[:, w:] == 5.0).all()

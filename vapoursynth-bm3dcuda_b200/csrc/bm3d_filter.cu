@@ -910,62 +910,73 @@ __global__ void __launch_bounds__(kAggThreads) aggregate_batch_kernel(AggregateB
     }
 }
 
-// One V-pixel quad (or single pixel) per thread; the stacks of up to 5 slots are
-// loaded before the first sum needs them.
-template <int V>
-__global__ void __launch_bounds__(128) vaggregate_kernel(VAggregateParams p) {
-    const int x = (blockIdx.x * blockDim.x + threadIdx.x) * V;
+// The stack of slot i of output frame n at (x, y), with replication padding at the
+// clip ends (source/source.cpp:832-836); its weight plane lies p.height rows below.
+__device__ __forceinline__ const float *vaggregate_slot(const VAggregateParams &p, int n, int i,
+                                                        int x, int y) {
+    const int s = min(max(2 * p.radius - i, n - p.num_frames + 1 + p.radius), n + p.radius);
+    const float *f = p.base ? p.base + (size_t)min(max(n - p.radius + i, 0), p.num_frames - 1) *
+                                           p.raw_frame_floats
+                            : p.vf[i];
+    return f + ((size_t)s * 2 * p.height + y) * p.raw_stride + x;
+}
+
+__global__ void vaggregate_kernel(VAggregateParams p) {
+    const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y;
     const int k = blockIdx.z;
     if (x >= p.width) return;
-    const int n = p.n0 + k;
+    const int tw = 2 * p.radius + 1;
+    float sw = 0.0f, sv = 0.0f;
+    for (int i = 0; i < tw; ++i) {
+        const float *a = vaggregate_slot(p, p.n0 + k, i, x, y);
+        sv = __fadd_rn(sv, a[0]);
+        sw = __fadd_rn(sw, a[(size_t)p.height * p.raw_stride]);
+    }
+    p.dst[k * p.dst_plane_stride + (size_t)y * p.dst_stride + x] = __fdiv_rn(sv, sw);
+}
+
+// Four pixels per thread; the stacks of up to 5 slots are loaded before the first
+// sum needs them.
+__global__ void __launch_bounds__(128) vaggregate_quad_kernel(VAggregateParams p) {
+    const int x = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    const int y = blockIdx.y;
+    const int k = blockIdx.z;
+    if (x >= p.width) return;
     const int tw = 2 * p.radius + 1;
     const size_t slab = (size_t)p.height * p.raw_stride;
-    auto stack = [&](int i) {
-        // replication padding at the clip ends (source/source.cpp:832-836)
-        const int s = min(max(2 * p.radius - i, n - p.num_frames + 1 + p.radius), n + p.radius);
-        const float *f = p.base ? p.base + (size_t)min(max(n - p.radius + i, 0), p.num_frames - 1) *
-                                              p.raw_frame_floats
-                                : p.vf[i];
-        return f + 2 * (size_t)s * slab + (size_t)y * p.raw_stride + x;
-    };
-    float sv[V] = {}, sw[V] = {};
+    float sv[4] = {}, sw[4] = {};
     for (int i0 = 0; i0 < tw; i0 += 5) {
-        float a[5][V], w[5][V];
+        float4 a[5], w[5];
 #pragma unroll
         for (int j = 0; j < 5; ++j) {
             if (i0 + j >= tw) break;
-            const float *src = stack(i0 + j);
-            if constexpr (V == 4) {
-                const float4 u = __ldg(reinterpret_cast<const float4 *>(src));
-                const float4 t = __ldg(reinterpret_cast<const float4 *>(src + slab));
-                a[j][0] = u.x; a[j][1] = u.y; a[j][2] = u.z; a[j][3] = u.w;
-                w[j][0] = t.x; w[j][1] = t.y; w[j][2] = t.z; w[j][3] = t.w;
-            } else {
-                a[j][0] = __ldg(src);
-                w[j][0] = __ldg(src + slab);
-            }
+            const float *src = vaggregate_slot(p, p.n0 + k, i0 + j, x, y);
+            a[j] = __ldg(reinterpret_cast<const float4 *>(src));
+            w[j] = __ldg(reinterpret_cast<const float4 *>(src + slab));
         }
 #pragma unroll
         for (int j = 0; j < 5; ++j) {
             if (i0 + j >= tw) break;
-#pragma unroll
-            for (int c = 0; c < V; ++c) {
-                sv[c] = __fadd_rn(sv[c], a[j][c]);
-                sw[c] = __fadd_rn(sw[c], w[j][c]);
-            }
+            sv[0] = __fadd_rn(sv[0], a[j].x);
+            sv[1] = __fadd_rn(sv[1], a[j].y);
+            sv[2] = __fadd_rn(sv[2], a[j].z);
+            sv[3] = __fadd_rn(sv[3], a[j].w);
+            sw[0] = __fadd_rn(sw[0], w[j].x);
+            sw[1] = __fadd_rn(sw[1], w[j].y);
+            sw[2] = __fadd_rn(sw[2], w[j].z);
+            sw[3] = __fadd_rn(sw[3], w[j].w);
         }
     }
     float *dst = p.dst + k * p.dst_plane_stride + (size_t)y * p.dst_stride + x;
-    float q[V];
+    float q[4];
 #pragma unroll
-    for (int c = 0; c < V; ++c) q[c] = __fdiv_rn(sv[c], sw[c]);
-    if (V == 4 && x + 4 <= p.width) {
-        *reinterpret_cast<float4 *>(dst) = make_float4(q[0], q[V > 1 ? 1 : 0], q[V > 2 ? 2 : 0],
-                                                       q[V > 3 ? 3 : 0]);
+    for (int c = 0; c < 4; ++c) q[c] = __fdiv_rn(sv[c], sw[c]);
+    if (x + 4 <= p.width) {
+        *reinterpret_cast<float4 *>(dst) = make_float4(q[0], q[1], q[2], q[3]);
     } else {
 #pragma unroll
-        for (int c = 0; c < V; ++c)
+        for (int c = 0; c < 4; ++c)
             if (x + c < p.width) dst[c] = q[c];
     }
 }
@@ -1156,21 +1167,25 @@ cudaError_t launch_aggregate(const AggregateParams &p, cudaStream_t stream) {
 
 cudaError_t launch_vaggregate(const VAggregateParams &p, cudaStream_t stream) {
     if (p.nout == 0) return cudaSuccess;
-    // quads where every row of every stack starts on 16 bytes (rows then have
-    // room for the last quad, the stride being a multiple of 4)
+    // Quads where every row of every stack starts on 16 bytes (rows then have room
+    // for the last quad, the stride being a multiple of 4) and is wider than a block of
+    // single pixels: below that both have as many blocks, and a quad's thread four times
+    // the work. (One frame, single pixels / quads, us: 1920x1080, radius 2 18.6 / 10.4, 3 26.8
+    // / 22.7; 160x2000, radius 3 7.4 / 6.3; 64x2000, radius 3 5.1 / 6.2.)
     unsigned long long align = reinterpret_cast<unsigned long long>(p.dst) |
                                reinterpret_cast<unsigned long long>(p.base);
     if (!p.base)
         for (int i = 0; i < 2 * p.radius + 1; ++i)
             align |= reinterpret_cast<unsigned long long>(p.vf[i]);
-    const bool quads = align % 16 == 0 && p.raw_stride % 4 == 0 && p.dst_stride % 4 == 0 &&
-                       p.raw_frame_floats % 4 == 0 && p.dst_plane_stride % 4 == 0;
+    const bool quads = p.width > 128 && align % 16 == 0 && p.raw_stride % 4 == 0 &&
+                       p.dst_stride % 4 == 0 && p.raw_frame_floats % 4 == 0 &&
+                       p.dst_plane_stride % 4 == 0;
     const int per_block = quads ? 512 : 128;
     const dim3 block(128), grid((p.width + per_block - 1) / per_block, p.height, p.nout);
     if (quads)
-        vaggregate_kernel<4><<<grid, block, 0, stream>>>(p);
+        vaggregate_quad_kernel<<<grid, block, 0, stream>>>(p);
     else
-        vaggregate_kernel<1><<<grid, block, 0, stream>>>(p);
+        vaggregate_kernel<<<grid, block, 0, stream>>>(p);
     return cudaGetLastError();
 }
 
